@@ -1,18 +1,14 @@
-// Axis passes on the tensor cores for large cubic grids (n = 96, 128), where the
-// whole-contour kernels do not fit in shared memory: one persistent launch per pass
-// (z, y or x) over both contour chains, the axis operator resident in shared memory
-// (even/odd form when centrosymmetric), DMMA tiles from the contour kernel
-// (row_op_ct / col_op_ct; two even/odd levels, row_op_eo2 / col_op_eo2, for 128-point
-// PMMM axes), and the next tile prefetched into registers while the current one is on
-// the tensor cores.  The Boltzmann factor exp(-w ds/2) of the
-// contour step is applied on the z-pass input (pre) and the x-pass output (post),
-// as in the per-axis SIMT kernels (axis_kernels.cuh) these replace for such grids.
+// FP32 axis passes on the tensor cores (3xTF32 split products) for large cubic grids (n = 96,
+// 128): one persistent launch per pass (z, y or x) over both contour chains, the axis operator
+// resident in shared memory (even/odd form when centrosymmetric), the tile routines of the
+// FP32 contour kernel (row_op_f32 / col_op_f32), and the next tile prefetched into registers
+// while the current one is on the tensor cores.  The Boltzmann factor exp(-w ds/2) of the
+// contour step is applied on the z-pass input (pre) and the x-pass output (post), as in the
+// per-axis SIMT kernels (axis_kernels.cuh).
 //
-//   z pass: rows of n contiguous values, tile = kRowsZ rows x n      (row_op_ct)
-//   y pass: for one x, tile = n (y) x kColsYX (z) with row stride n   (col_op_ct)
-//   x pass: for one y, tile = n (x) x kColsYX (z) with row stride n^2 (col_op_ct)
-// FP64 runs on DMMA (axis_dmma_kernel); the FP32 precision form on 3xTF32 split products
-// (axis_tf32_kernel, row_op_f32 / col_op_f32).
+//   z pass: rows of n contiguous values, tile = kRowsZ rows x n
+//   y pass: for one x, tile = n (y) x kColsYX (z) with row stride n
+//   x pass: for one y, tile = n (x) x kColsYX (z) with row stride n^2
 #pragma once
 #include <cuda_runtime.h>
 
@@ -43,20 +39,6 @@ __device__ __forceinline__ unsigned long long l2_policy(bool last) {
     else asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
     return p;
 }
-__device__ __forceinline__ double2 ld_cg_policy(const double* a, unsigned long long pol) {
-    double2 v;
-    asm volatile("ld.global.cg.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(a), "l"(pol));
-    return v;
-}
-__device__ __forceinline__ double2 ld_nc_policy(const double* a, unsigned long long pol) {
-    double2 v;
-    asm volatile("ld.global.nc.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;" : "=d"(v.x), "=d"(v.y) : "l"(a), "l"(pol));
-    return v;
-}
-__device__ __forceinline__ void st_cg_policy(double* a, double2 v, unsigned long long pol) {
-    asm volatile("st.global.cg.L2::cache_hint.v2.f64 [%0], {%1, %2}, %3;" ::"l"(a), "d"(v.x), "d"(v.y), "l"(pol)
-                 : "memory");
-}
 __device__ __forceinline__ float4 ld_cg_policy(const float* a, unsigned long long pol) {
     float4 v;
     asm volatile("ld.global.cg.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
@@ -75,34 +57,7 @@ __device__ __forceinline__ void st_cg_policy(float* a, float4 v, unsigned long l
                  : "memory");
 }
 
-struct AxisPassD {
-    const double* in[2];
-    double* out[2];
-    const double* pre[2];   // z pass: input *= pre (nullptr: none)
-    const double* post[2];  // x pass: output *= post (nullptr: none)
-    const double* op;       // this axis' packed operator (AxisShape<N, EO> or AxisShapeEO2<N> layout)
-    int nchain;
-    int hints;              // 1: L2 eviction priorities on the pass traffic (see l2_policy)
-    int discard_in;         // 1: the input is dead once read (a triplet intermediate): drop its
-                            // L2 lines after the tile is loaded (y and x passes)
-};
-
-template <int N, bool EO, bool EO2 = false>
-struct AxisDmmaShape {
-    static_assert(!EO2 || (EO && N == 128), "two even/odd levels: 128-point even/odd axes");
-    static constexpr int OP_VALUES = EO2 ? AxisShapeEO2<N>::SIZE : AxisShape<N, EO>::SIZE;
-    static constexpr int OPS = (OP_VALUES + 15) & ~15;
-    static constexpr int LFZ = N + 4;       // z tile: kRowsZ x N
-    static constexpr int LFC = kColsYX + 4;  // y/x tile: N x kColsYX
-    static constexpr int TILE = (N * LFC > kRowsZ * LFZ ? N * LFC : kRowsZ * LFZ);
-    static constexpr int TILE_PAD = (TILE + 15) & ~15;
-    static constexpr size_t SMEM = (size_t)(OPS + 2 * TILE_PAD) * sizeof(double);
-    static constexpr int PER_THREAD = N * kColsYX / 2 / kContourThreads;  // double2 per thread and tile
-    static_assert(N * kColsYX == kRowsZ * N, "z and y/x tiles hold the same number of values");
-    static_assert(PER_THREAD * 2 * kContourThreads == N * kColsYX, "tile not a multiple of the block");
-};
-
-// element (r, c) of tile `t` (double2 granularity: c even) and its global offset
+// element (r, c) of tile `t` and its global offset
 template <int N, int AX>
 struct AxisTiling {
     static constexpr long long M = (long long)N * N * N;
@@ -117,102 +72,6 @@ struct AxisTiling {
     static constexpr int ROW_LEN = AX == 2 ? N : kColsYX;  // values per tile row
 };
 
-template <int N, bool EO, int AX, bool EO2 = false>
-__global__ void __launch_bounds__(kContourThreads, 1) axis_dmma_kernel(const AxisPassD p) {
-    using S = AxisDmmaShape<N, EO, EO2>;
-    using TL = AxisTiling<N, AX>;
-    constexpr int LF = AX == 2 ? S::LFZ : S::LFC;
-    constexpr int RL = TL::ROW_LEN;
-    constexpr int PT = S::PER_THREAD;
-    extern __shared__ __align__(16) double axs[];
-    double* sop = axs;
-    double* F = axs + S::OPS;
-    double* G = F + S::TILE_PAD;
-    op_copy_async(sop, p.op, S::OP_VALUES);
-
-    const int tiles = p.nchain * TL::TILES_PER_CHAIN;
-    const unsigned long long pol_first = l2_policy(false), pol_last = l2_policy(true);
-    double2 v[PT], w[PT];
-    // fetch tile t into registers (input x pre for the z pass; post for the x pass)
-    auto fetch = [&](int t) {
-        const int c = t / TL::TILES_PER_CHAIN;
-        const long long o = TL::origin(t - c * TL::TILES_PER_CHAIN);
-        const double* in = p.in[c] + o;
-        const double* aux = AX == 2 ? p.pre[c] : (AX == 0 ? p.post[c] : nullptr);
-#pragma unroll
-        for (int k = 0; k < PT; ++k) {
-            const int e = (k * kContourThreads + threadIdx.x) * 2;
-            const int r = e / RL, cc = e - r * RL;
-            const long long g = r * TL::ROW_STRIDE + cc;
-            if (p.hints) {
-                v[k] = ld_cg_policy(in + g, pol_first);
-                if (aux) w[k] = ld_nc_policy(aux + o + g, pol_last);
-            } else {
-                v[k] = __ldcg(reinterpret_cast<const double2*>(in + g));
-                if (aux) w[k] = __ldg(reinterpret_cast<const double2*>(aux + o + g));
-            }
-        }
-    };
-    int t = blockIdx.x;
-    if (t < tiles) fetch(t);  // in flight with the operator copies
-    cp_async_wait_all();      // the operator; the loop's first barrier publishes it
-    for (; t < tiles; t += gridDim.x) {
-        const int c = t / TL::TILES_PER_CHAIN;
-        const long long o = TL::origin(t - c * TL::TILES_PER_CHAIN);
-        const bool pre = AX == 2 && p.pre[c] != nullptr;
-        const bool post = AX == 0 && p.post[c] != nullptr;
-        __syncthreads();  // the previous tile's G has been stored, F may be overwritten
-#pragma unroll
-        for (int k = 0; k < PT; ++k) {
-            const int e = (k * kContourThreads + threadIdx.x) * 2;
-            const int r = e / RL, cc = e - r * RL;
-            double2 x = v[k];
-            if (pre) {
-                x.x *= w[k].x;
-                x.y *= w[k].y;
-            }
-            *reinterpret_cast<double2*>(F + r * LF + cc) = x;
-        }
-        double2 wpost[PT];
-        if (post) {
-#pragma unroll
-            for (int k = 0; k < PT; ++k) wpost[k] = w[k];
-        }
-        __syncthreads();
-        if (AX != 2 && p.discard_in) {
-            // every load of this tile has returned (its values are in F): drop the input's
-            // lines, two 128-byte lines per tile row of kColsYX doubles
-            constexpr int LINES = N * (kColsYX * (int)sizeof(double) / 128);
-            if (threadIdx.x < LINES) {
-                const int r = threadIdx.x / (LINES / N), h = threadIdx.x - r * (LINES / N);
-                l2_discard_line(p.in[c] + o + r * TL::ROW_STRIDE + h * (128 / (int)sizeof(double)));
-            }
-        }
-        if (t + (int)gridDim.x < tiles) fetch(t + gridDim.x);  // in flight during the MMAs
-        if constexpr (AX == 2) {
-            if constexpr (EO2) row_op_eo2<kRowsZ, N, LF>(F, G, sop);
-            else row_op_ct<kRowsZ, N, LF, EO>(F, G, sop);
-        } else {
-            if constexpr (EO2) col_op_eo2<N, kColsYX, LF, kToSmem>(F, ColOut{G, 0}, sop);
-            else col_op_ct<N, kColsYX, LF, EO>(F, G, sop);
-        }
-        __syncthreads();
-        double* out = p.out[c] + o;
-#pragma unroll
-        for (int k = 0; k < PT; ++k) {
-            const int e = (k * kContourThreads + threadIdx.x) * 2;
-            const int r = e / RL, cc = e - r * RL;
-            double2 y = *reinterpret_cast<const double2*>(G + r * LF + cc);
-            if (post) {
-                y.x *= wpost[k].x;
-                y.y *= wpost[k].y;
-            }
-            if (p.hints) st_cg_policy(out + r * TL::ROW_STRIDE + cc, y, pol_last);
-            else __stcg(reinterpret_cast<double2*>(out + r * TL::ROW_STRIDE + cc), y);
-        }
-    }
-}
-
 // ---- FP32 (3xTF32) form ---------------------------------------------------------
 struct AxisPassF {
     const float* in[2];
@@ -221,8 +80,9 @@ struct AxisPassF {
     const float* post[2];
     const float* op;  // this axis' packed TF32 hi/lo operator (AxisShapeF<N, EO> layout)
     int nchain;
-    int hints;        // as AxisPassD::hints
-    int discard_in;   // as AxisPassD::discard_in
+    int hints;        // 1: L2 eviction priorities on the pass traffic (see l2_policy)
+    int discard_in;   // 1: the input is dead once read (a triplet intermediate): drop its L2 lines after
+                      // the tile is loaded (y and x passes)
 };
 
 template <int N, bool EO>
@@ -300,7 +160,7 @@ __global__ void __launch_bounds__(kContourThreads) axis_tf32_kernel(const AxisPa
             for (int k = 0; k < PT; ++k) wpost[k] = w[k];
         }
         __syncthreads();
-        if (AX != 2 && p.discard_in) {  // as in axis_dmma_kernel: one 128-byte line per tile row
+        if (AX != 2 && p.discard_in) {  // one 128-byte line per tile row, every load of the tile has returned
             static_assert(kColsYX * sizeof(float) == 128, "one line per FP32 tile row");
             if (threadIdx.x < N) l2_discard_line(p.in[c] + o + threadIdx.x * TL::ROW_STRIDE);
         }

@@ -68,18 +68,40 @@ __device__ __forceinline__ double block_max(double v, double* sh) {
     return r;
 }
 
+// Point order of the contour (slices and Boltzmann factors).  The fields are always in the
+// solver's storage order; the FP64 contour of a 3m solver without translations is kept in the
+// order of positions along the half lines, in which its operators are the PMMM ones (on = 1):
+// storage index s of an axis of n points is position 2 s, or 2 (n - 1 - s) + 1 beyond the middle.
+struct PointOrder {
+    int on = 0, nx = 0, ny = 0, nz = 0;
+    __device__ __forceinline__ static int position(int s, int n) { return 2 * s < n ? 2 * s : 2 * (n - 1 - s) + 1; }
+    __device__ __forceinline__ static int storage(int j, int n) { return (j & 1) ? n - 1 - (j >> 1) : (j >> 1); }
+    // contour index of field point i, and the reverse
+    __device__ __forceinline__ long long to_contour(long long i) const {
+        if (!on) return i;
+        const int z = (int)(i % nz), y = (int)((i / nz) % ny), x = (int)(i / ((long long)ny * nz));
+        return ((long long)position(x, nx) * ny + position(y, ny)) * nz + position(z, nz);
+    }
+    __device__ __forceinline__ long long to_field(long long i) const {
+        if (!on) return i;
+        const int z = (int)(i % nz), y = (int)((i / nz) % ny), x = (int)(i / ((long long)ny * nz));
+        return ((long long)storage(x, nx) * ny + storage(y, ny)) * nz + storage(z, nz);
+    }
+};
+
 template <typename T>
 __global__ void prep_kernel(const double* __restrict__ wA, const double* __restrict__ wB,
                             double* __restrict__ ksi, T* __restrict__ wAds, T* __restrict__ wBds,
                             T* __restrict__ q_first, T* __restrict__ qc_last, double xN, double ds,
-                            long long M) {
+                            long long M, PointOrder po) {
     const double index = -ds / 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M;
          i += (long long)gridDim.x * blockDim.x) {
         const double a = wA[i], b = wB[i];
         ksi[i] = 0.5 * (a + b - xN);
-        wAds[i] = (T)(1. * exp(index * a));
-        wBds[i] = (T)(1. * exp(index * b));
+        const long long j = po.to_contour(i);
+        wAds[j] = (T)(1. * exp(index * a));
+        wBds[j] = (T)(1. * exp(index * b));
         q_first[i] = T(1);
         qc_last[i] = T(1);
     }
@@ -152,7 +174,7 @@ __device__ __forceinline__ void phi_point_pair(const T* __restrict__ q, const T*
 template <typename T>
 __global__ void phi_kernel(const T* __restrict__ q, const T* __restrict__ qc, double* __restrict__ phiA,
                            double* __restrict__ phiB, const IterState* st, double fA, long long NsA,
-                           long long NsB, long long M) {
+                           long long NsB, long long M, PointOrder po) {
     const double Q = st->Q;
     const double fB = 1 - fA;
     const double cA = fA / (NsA * Q);
@@ -172,8 +194,9 @@ __global__ void phi_kernel(const T* __restrict__ q, const T* __restrict__ qc, do
                 const long long u = NsA + s;
                 b += factor * (double)q[u * M + i] * (double)qc[u * M + i];
             }
-            phiA[i] = a;
-            phiB[i] = b;
+            const long long f = po.to_field(i);
+            phiA[f] = a;
+            phiB[f] = b;
         }
         return;
     }
@@ -184,8 +207,16 @@ __global__ void phi_kernel(const T* __restrict__ q, const T* __restrict__ qc, do
         double a0 = 0.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
         phi_point_pair<T>(q, qc, M, i, 0, NsA, cA, a0, a1);
         phi_point_pair<T>(q, qc, M, i, NsA, NsB, cB, b0, b1);
-        *reinterpret_cast<double2*>(phiA + i) = make_double2(a0, a1);
-        *reinterpret_cast<double2*>(phiB + i) = make_double2(b0, b1);
+        if (po.on) {
+            const long long f0 = po.to_field(i), f1 = po.to_field(i + 1);
+            phiA[f0] = a0;
+            phiA[f1] = a1;
+            phiB[f0] = b0;
+            phiB[f1] = b1;
+        } else {
+            *reinterpret_cast<double2*>(phiA + i) = make_double2(a0, a1);
+            *reinterpret_cast<double2*>(phiB + i) = make_double2(b0, b1);
+        }
     }
 }
 
@@ -200,7 +231,7 @@ template <typename T>
 __global__ void phi_fused_finish_kernel(const double* __restrict__ acc, const T* __restrict__ q,
                                         const T* __restrict__ qc, double* __restrict__ phiA,
                                         double* __restrict__ phiB, const IterState* st, double fA, long long NsA,
-                                        long long NsB, int n) {
+                                        long long NsB, int n, PointOrder po) {
     const long long n2 = (long long)n * n, M = n2 * n, U = NsA + NsB;
     const double Q = st->Q;
     const double cA = fA / (NsA * Q), cB = (1 - fA) / (NsB * Q);
@@ -227,8 +258,9 @@ __global__ void phi_fused_finish_kernel(const double* __restrict__ acc, const T*
             if (s <= NsA) a += (s == 0 || s == NsA ? 0.5 : 1.0) * w;
             if (s >= NsA) b += (s == NsA || s == U ? 0.5 : 1.0) * w;
         }
-        phiA[i] = cA * a;
-        phiB[i] = cB * b;
+        const long long f = po.to_field(i);
+        phiA[f] = cA * a;
+        phiB[f] = cB * b;
     }
 }
 

@@ -22,9 +22,11 @@
 #include "axis_dmma.cuh"
 #include "axis_fft.cuh"
 #include "axis_kernels.cuh"
+#include "axis_mma.cuh"
 #include "contour_kernel.cuh"
 #include "contour_batch.cuh"
 #include "contour_cluster_f32.cuh"
+#include "contour_step.cuh"
 #include "contour_kernel_f32.cuh"
 #include "field_kernels.cuh"
 #include "operators.h"
@@ -158,7 +160,7 @@ struct OpsSet {
     // even/odd axis E then O (h x h, leading dimension h+4), else A (n x n, n+4)
     std::vector<double> h_packed;
     DevBuf<double> d_packed;
-    // two even/odd levels (PMMM, n = 64 or 128 on every axis): per axis [EE | EO | O]
+    // two even/odd levels (PMMM and 3m, n = 64 on every axis): per axis [EE | EO | O]
     // (AxisShapeEO2), x then y then z
     std::vector<double> h_packed2;
     DevBuf<double> d_packed2;
@@ -182,6 +184,22 @@ struct OpsSet {
     DevBuf<double2> d_fft_tw[3];
     DevBuf<float> f_fft_g[3];   // the same tables rounded to FP32 (precision form)
     DevBuf<float2> f_fft_tw[3];
+    // FP64 tensor-core axis passes (axis_mma.cuh): the packed blocks of the three axes, one
+    // allocation; mode -1: an axis beyond kMmaMaxN
+    struct Mma {
+        int mode = -1, perm = 0, n = 0;
+        size_t off = 0;
+    };
+    Mma mma[3], dmma[3];
+    DevBuf<double> d_mma, d_dmma;
+    static std::vector<const Mma*> before(const Mma* axes, int ax) {
+        std::vector<const Mma*> e;
+        for (int a = 0; a < ax; ++a) e.push_back(&axes[a]);
+        return e;
+    }
+    // 3m without translations, axes within kMmaMaxN: the FP64 contour is kept in position order
+    // (PointOrder), and the packed FP64 operators of the contour kernels are in that order
+    bool pos_order = false;
     // cell-length derivatives dA/dL of the three axis operators (built on first use)
     DevBuf<double> d_dop[3], d_dopT[3];
     bool have_dop = false;
@@ -345,11 +363,12 @@ AxisFftFn<R> axis_fft_kernel_for(int n, int nf, int ext, size_t* smem) {
 }
 
 // Which form runs the per-axis passes: CRYSSCFT_AXIS_FORM=fft or =dense forces one (for
-// measurements and tests); by default the FFT passes run wherever they exist except where
-// the tensor-core passes were measured faster (scft_solver_s::tensor_axis_passes: PMMM
-// grids they cover, and P1 iterations).  Per triplet on one B200: 256-point P1 axes 0.28 ms
-// by FFT against 2.99 ms by the SIMT GEMMs; 128-point PMMM axes 65 us by FFT against 56 us
-// by DMMA.
+// measurements and tests).  By default FP64 axes of up to kMmaMaxN points take the tensor-core
+// passes (axis_mma.cuh), longer ones the FFT where it exists (256-point P1 axes: 0.28 ms a
+// triplet against 2.99 ms by the SIMT GEMMs); FP32 triplets take the FFT where it exists except
+// on the grids of scft_solver_s::tf32_axis_passes.  FP64 per triplet on one B200, three calls of
+// this library among others: 64^3 PMMM 12 us against 30 us by FFT, 45 x 40 x 54 P1 15 us against
+// 37 us by the SIMT GEMMs, 128^3 PMMM 44 us, 3m 43 us, P1 40 us against 65, 68 and 50 us by FFT.
 int axis_form_override() {
     const char* e = getenv("CRYSSCFT_AXIS_FORM");
     return !e ? 0 : (e[0] == 'f' ? 1 : (e[0] == 'd' ? 2 : 0));
@@ -393,10 +412,10 @@ void pack_operator(const std::vector<long double>& A, int n, OpsSet& s, int axis
 }
 
 // Append one axis operator in the two-level even/odd form when its even half is itself
-// centrosymmetric (PMMM) and n is 64 (whole-contour kernel) or 128 (axis passes); returns
+// centrosymmetric (PMMM, 3m in position order) and n is 64 (whole-contour kernel); returns
 // false (and appends nothing) otherwise.
 bool pack_operator_eo2(const std::vector<long double>& A, int n, OpsSet& s) {
-    if (n != 64 && n != 128) return false;
+    if (n != 64) return false;
     const int h = n / 2, h2 = n / 4;
     std::vector<long double> E((size_t)h * h), O((size_t)h * h);
     for (int i = 0; i < h; ++i)
@@ -426,6 +445,83 @@ bool pack_operator_eo2(const std::vector<long double>& A, int n, OpsSet& s) {
     for (int i = 0; i < h; ++i)
         for (int j = 0; j < h; ++j) OO[(size_t)i * ld + j] = (double)O[(size_t)i * h + j];
     return true;
+}
+
+// the matrix A of a 3m axis (storage order) in position order
+std::vector<long double> position_order(const std::vector<long double>& A, int n) {
+    auto at = [&](int j) { return (j & 1) ? n - 1 - (j >> 1) : (j >> 1); };
+    std::vector<long double> B(A.size());
+    for (int i = 0; i < n; ++i)
+        for (int j = 0; j < n; ++j) B[(size_t)i * n + j] = A[(size_t)at(i) * n + at(j)];
+    return B;
+}
+
+bool same(long double a, long double b) { return fabsl(a - b) <= 1e-17L * (1.0L + fabsl(a)); }
+
+// Append one axis operator (n <= kMmaMaxN) in the block form of axis_mma.cuh its symmetry
+// allows.  perm: A is in 3m order (the pass reads and writes its points in that order).
+// earlier: the axes already packed into the same buffer.
+void pack_operator_mma(const std::vector<long double>& A0, int n, bool perm, OpsSet::Mma& m, std::vector<double>& packed,
+                       const std::vector<const OpsSet::Mma*>& earlier) {
+    m = OpsSet::Mma{};
+    if (n > kMmaMaxN) return;
+    m.n = n;
+    m.perm = perm ? 1 : 0;
+    auto at = [&](int j) { return !perm ? j : ((j & 1) ? n - 1 - (j >> 1) : (j >> 1)); };
+    auto A = [&](int i, int j) { return A0[(size_t)at(i) * n + at(j)]; };
+    bool centro = true;
+    for (int i = 0; centro && i < n; ++i)
+        for (int j = 0; centro && j < n; ++j) centro = same(A(i, j), A(n - 1 - i, n - 1 - j));
+    const int half = n / 2;
+    // two-level forms: only for the lengths with a specialised kernel (64, 96, 128)
+    bool eo2 = centro && n % 32 == 0 && n >= 64, circ = eo2;
+    auto E = [&](int i, int j) { return (A(i, j) + A(i, n - 1 - j)) / 2; };
+    for (int i = 0; i < half && (eo2 || circ); ++i)
+        for (int j = 0; j < half && (eo2 || circ); ++j) {
+            eo2 = eo2 && same(E(i, j), E(half - 1 - i, half - 1 - j));
+            circ = circ && same(A(i, j), A(i + half, j + half)) && same(A(i, j + half), A(i + half, j)) &&
+                   same(A(i, j), A(half - 1 - i, half - 1 - j)) &&
+                   same(A(i, j + half), A(half - 1 - i, n - 1 - j));
+        }
+    m.mode = circ ? kCirc4 : (eo2 ? kEo2 : (centro ? kEo1 : kFull));
+    const AxisBlocks b(m.mode, n);
+    m.off = packed.size();
+    packed.resize(m.off + (size_t)b.count, 0.0);
+    double* o = packed.data() + m.off;
+    const size_t blk = (size_t)b.hp * b.ld;
+    for (int i = 0; i < b.h; ++i)
+        for (int j = 0; j < b.h; ++j) {
+            const size_t e = (size_t)i * b.ld + j;
+            if (m.mode == kFull) {
+                o[e] = (double)A(i, j);
+            } else if (m.mode == kEo1) {
+                const bool mid = 2 * j == n - 1;  // u holds the middle point twice
+                o[e] = (double)(mid ? A(i, j) / 2 : E(i, j));
+                o[blk + e] = mid ? 0.0 : (double)((A(i, j) - A(i, n - 1 - j)) / 2);
+            } else if (m.mode == kEo2) {
+                o[e] = (double)((E(i, j) + E(i, half - 1 - j)) / 2);
+                o[blk + e] = (double)((E(i, j) - E(i, half - 1 - j)) / 2);
+            } else {
+                for (int s = 0; s < 2; ++s) {  // the circulant and the skew-circulant half
+                    const long double a = (A(i, j) + (s ? -1 : 1) * A(i, j + half)) / 2;
+                    const long double c = (A(i, half - 1 - j) + (s ? -1 : 1) * A(i, n - 1 - j)) / 2;
+                    o[(size_t)(2 * s) * blk + e] = (double)((a + c) / 2);
+                    o[(size_t)(2 * s + 1) * blk + e] = (double)((a - c) / 2);
+                }
+            }
+        }
+    if (m.mode == kEo2)
+        for (int i = 0; i < half; ++i)
+            for (int j = 0; j < half; ++j)
+                o[2 * blk + (size_t)i * b.ldo + j] = (double)((A(i, j) - A(i, n - 1 - j)) / 2);
+    // axes with equal operators (cubic cells) share one copy
+    for (const OpsSet::Mma* e : earlier)
+        if (e->mode == m.mode && e->n == n && e->perm == m.perm &&
+            std::equal(packed.begin() + (long)m.off, packed.end(), packed.begin() + (long)e->off)) {
+            packed.resize(m.off);
+            m.off = e->off;
+            break;
+        }
 }
 
 int upload_operator(const std::vector<long double>& A, int n, OpsSet& s, int axis) {
@@ -488,29 +584,53 @@ cudaError_t launch_axis(const AxisPass<T>& p, int nchain, bool contiguous, cudaS
     return launch_strided_bm<T, 64>(p, nchain, st);
 }
 
-using AxisDmmaFn = void (*)(const AxisPassD);
+using AxisMmaFn = void (*)(const AxisMmaPass);
 
-// The FP64 tensor-core axis pass for a cubic grid of side n (96 or 128); nullptr if none.
-// eo2: the operators are in the two-level even/odd form (AxisShapeEO2, n = 128).
-AxisDmmaFn axis_dmma_kernel_for(int n, int eo, int ax, size_t* smem, bool eo2 = false) {
-    if (eo2 && eo && n == 128) {
-        *smem = AxisDmmaShape<128, true, true>::SMEM;
-        return ax == 0 ? axis_dmma_kernel<128, true, 0, true>
-                       : (ax == 1 ? axis_dmma_kernel<128, true, 1, true> : axis_dmma_kernel<128, true, 2, true>);
+// The FP64 tensor-core pass of an axis of length n (<= kMmaMaxN) in block form `mode`.
+AxisMmaFn axis_mma_kernel_for(int mode, int n, bool row) {
+#define CRYSSCFT_MMA(M_, NC_, NMAX_, ML_) \
+    return row ? axis_mma_kernel<M_, true, NC_, NMAX_, ML_> : axis_mma_kernel<M_, false, NC_, NMAX_, ML_>;
+    if (mode == kEo2) {
+        if (n == 128) CRYSSCFT_MMA(kEo2, 128, 128, 2)
+        if (n == 96) CRYSSCFT_MMA(kEo2, 96, 96, 2)
+        if (n == 64) CRYSSCFT_MMA(kEo2, 64, 64, 1)
     }
-#define CRYSSCFT_AXD(N, E)                                            \
-    {                                                                 \
-        *smem = AxisDmmaShape<N, E>::SMEM;                            \
-        return ax == 0 ? axis_dmma_kernel<N, E, 0>                    \
-                       : (ax == 1 ? axis_dmma_kernel<N, E, 1> : axis_dmma_kernel<N, E, 2>); \
+    if (mode == kCirc4) {
+        if (n == 128) CRYSSCFT_MMA(kCirc4, 128, 128, 2)
+        if (n == 96) CRYSSCFT_MMA(kCirc4, 96, 96, 2)
+        if (n == 64) CRYSSCFT_MMA(kCirc4, 64, 64, 1)
     }
-    if (n == 128) {
-        if (eo) CRYSSCFT_AXD(128, true) else CRYSSCFT_AXD(128, false)
+    if (mode == kEo1) {
+        if (n <= 64) CRYSSCFT_MMA(kEo1, 0, 64, 1)
+        if (n <= 128) CRYSSCFT_MMA(kEo1, 0, 128, 2)
     }
-    if (n == 96) {
-        if (eo) CRYSSCFT_AXD(96, true) else CRYSSCFT_AXD(96, false)
+    if (mode == kFull) {
+        if (n <= 64) CRYSSCFT_MMA(kFull, 0, 64, 1)
+        if (n <= 128) CRYSSCFT_MMA(kFull, 0, 128, 2)
     }
-#undef CRYSSCFT_AXD
+#undef CRYSSCFT_MMA
+    return nullptr;
+}
+
+using ContourStepFn = void (*)(const ContourStepArgs);
+
+// The one-launch-per-step kernel for a cubic grid of side n whose axes are all in block form
+// `mode`; one_op: the three axes share one operator.  *smem 0: none.
+ContourStepFn contour_step_kernel_for(int mode, int n, bool one_op, int* threads, size_t* smem) {
+#define CRYSSCFT_STEP(M_, N_, ML_)                     \
+    if (mode == M_ && n == N_) {                       \
+        *threads = StepShape<M_, N_, ML_>::THREADS;    \
+        *smem = StepShape<M_, N_, ML_>::smem(one_op);  \
+        return contour_step_kernel<M_, N_, ML_>;       \
+    }
+    CRYSSCFT_STEP(kEo2, 128, 2)
+    CRYSSCFT_STEP(kEo2, 96, 1)
+    CRYSSCFT_STEP(kCirc4, 128, 2)
+    CRYSSCFT_STEP(kCirc4, 96, 1)
+    CRYSSCFT_STEP(kEo2, 64, 1)
+    CRYSSCFT_STEP(kCirc4, 64, 1)
+#undef CRYSSCFT_STEP
+    *smem = 0;
     return nullptr;
 }
 
@@ -633,6 +753,13 @@ ContourFn contour_kernel_for(int nx, int ny, int nz, const int eo[3]) {
 
 }  // namespace
 
+// One chain of contour steps over a store of slices: input slot slot0 + dir t of step t.
+struct ChainSpan {
+    double* q;
+    long long slot0;
+    int dir;
+};
+
 // ---------------------------------------------------------------------------
 // solver
 // ---------------------------------------------------------------------------
@@ -643,9 +770,7 @@ struct scft_solver_s {
     int users = 0;                 // iteration contexts (scft_diblock_t) built on this solver
     bool destroy_pending = false;  // scft_solver_destroy was called while users > 0
     int sms = 0;                   // multiprocessors of `device` (queried on first use)
-    size_t axis_dmma_smem_set = 0; // dynamic shared memory granted to the tensor-core axis passes
-    const void* axis_dmma_fn_set = nullptr;  // ... and to which kernel family (z pass)
-    size_t axis_tf32_smem_set = 0;
+    size_t axis_tf32_smem_set = 0;  // dynamic shared memory granted to the FP32 tensor-core axis passes
     size_t grid_log[3] = {0, 0, 0};
     size_t grid_phy[3] = {0, 0, 0};
     size_t M = 0;
@@ -678,81 +803,235 @@ struct scft_solver_s {
                 if (m3sym.half[a][b]) return false;
         return true;
     }
-    std::vector<const void*> fft_fn_set;  // FFT kernels granted their dynamic shared memory
+    // kernels of the axis passes granted their dynamic shared memory: (kernel, bytes) -> CTAs per SM
+    std::map<std::pair<const void*, size_t>, int> pass_ctas;
 
-    // whether the tensor-core axis passes (axis_dmma.cuh: FP64 DMMA; FP32: 3xTF32) run this
-    // grid by default, on a cubic grid with a side the kernels cover (96 or 128), from
-    // measurements on one B200: PMMM (two-level even/odd operators) always, 56 us against 65 us
-    // by FFT per 256^3 triplet; P1 for both chains of an iteration (128^3: 52.5 against 49.4
-    // iterations/s, precision form 69.7 against 62.1) but not for one chain (50 us by FFT
-    // against 58 us); never 3m (128-point axes: 68 us by FFT against 82 us per triplet, 36.6
-    // against 33.6 iterations/s at 256^3)
-    template <typename T>
-    bool tensor_axis_passes(int nchain) const {
-        const OpsSet* o = ops;
-        const int n = (int)grid_phy[0];
-        if (kind == SCFT_SOLVER_3M || (kind == SCFT_SOLVER_P1 && nchain < 2)) return false;
-        if (o->nterms != 1 || grid_phy[1] != grid_phy[0] || grid_phy[2] != grid_phy[0]) return false;
-        size_t smem = 0, stride = 0;
-        if constexpr (sizeof(T) == 8) {
-            if (o->eo[0] != o->eo[1] || o->eo[1] != o->eo[2]) return false;
-            return axis_dmma_kernel_for(n, o->eo[0], 2, &smem, o->eo2 && n == 128) != nullptr;
-        } else {
-            if (o->eo_f32[0] != o->eo_f32[1] || o->eo_f32[1] != o->eo_f32[2]) return false;
-            return axis_tf32_kernel_for(n, o->eo_f32[0], 2, &smem, &stride) != nullptr;
+    int grant_pass(const void* fn, int threads, size_t smem, int* grid) {
+        if (!sms) CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        int& per_sm = pass_ctas[{fn, smem}];
+        if (!per_sm) {
+            // the limit is the function's, shared by every solver: always the device's most
+            int dev_smem = 0;
+            cudaFuncAttributes fa{};
+            CK(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+            CK(cudaFuncGetAttributes(&fa, fn));
+            CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dev_smem - (int)fa.sharedSizeBytes));
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
+            if (per_sm < 1) per_sm = 1;
         }
+        *grid = sms * per_sm;
+        return SCFT_OK;
     }
 
-    // the three passes of a triplet by FFT (axis_fft.cuh); *done = false if an axis has no
-    // FFT form or the dense form is to run
-    template <typename T>
-    int triplet_fft(int nchain, const ChainIO<T> io[2], T* t1[2], T* t2[2], cudaStream_t st, bool* done) {
-        *done = false;
+    // One FP64 tensor-core pass along axis ax (axis_mma.cuh) of `stack` stacked fields per chain.
+    int mma_pass(int ax, const OpsSet::Mma& m, const double* ops_base, int nchain, const double* const in[2],
+                 double* const out[2], const double* const pre[2], const double* const post[2], long long stack,
+                 bool accum, bool discard_in, cudaStream_t st, bool in_positions = false) {
+        const bool row = ax == 2;
+        AxisMmaPass p{};
+        for (int c = 0; c < nchain; ++c) {
+            p.in[c] = in[c];
+            p.out[c] = out[c];
+            p.pre[c] = pre ? pre[c] : nullptr;
+            p.post[c] = post ? post[c] : nullptr;
+        }
+        p.op = ops_base + m.off;
+        p.op_count = AxisBlocks(m.mode, m.n).count;
+        p.n = m.n;
+        p.perm = in_positions ? 0 : m.perm;
+        p.accum = accum ? 1 : 0;
+        p.nchain = nchain;
+        const long long nx = (long long)grid_phy[0], ny = (long long)grid_phy[1], nz = (long long)grid_phy[2];
+        p.outer = stack * (ax == 2 ? nx * ny : (ax == 1 ? nx : 1));
+        p.inner = ax == 2 ? 1 : (ax == 1 ? nz : ny * nz);
+        p.discard_in = discard_in && !row && p.inner % kMmaLines == 0 ? 1 : 0;
+        const AxisMmaFn f = axis_mma_kernel_for(m.mode, m.n, row);
+        const size_t smem = axis_mma_smem(m.mode, m.n, row);
+        int grid = 1;
+        CKR(grant_pass((const void*)f, kMmaThreads, smem, &grid));
+        const long long lines = row ? p.outer : p.outer * p.inner;
+        grid = (int)std::min<long long>(grid, nchain * ((lines + kMmaLines - 1) / kMmaLines));
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(kMmaThreads);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        CK(cudaLaunchKernelEx(&cfg, f, p));
+        ++launches;
+        return SCFT_OK;
+    }
+
+    // dynamic shared memory of the one-launch-per-step kernel on this grid (contour_step.cuh), 0 if
+    // it does not apply: cubic, side 96 or 128, one block form on all axes, and room for the
+    // operators beside the tile (128-point PMMM and 3m axes: only if the three are equal)
+    size_t step_smem(int* threads = nullptr, ContourStepFn* fn = nullptr) {
         const OpsSet* o = ops;
-        if (o->nterms != 1) return SCFT_OK;
+        if (!o || o->nterms != 1 || axis_form_override() != 0) return 0;
+        if (grid_phy[0] != grid_phy[1] || grid_phy[1] != grid_phy[2]) return 0;
+        const OpsSet::Mma* m = o->mma;
+        if (m[0].mode != m[1].mode || m[1].mode != m[2].mode) return 0;
+        if (m[0].perm && !o->pos_order) return 0;
+        size_t smem = 0;
+        int th = 0;
+        const bool one_op = m[0].off == m[1].off && m[1].off == m[2].off;
+        const ContourStepFn f = contour_step_kernel_for(m[0].mode, (int)grid_phy[0], one_op, &th, &smem);
+        int dev_smem = 0;
+        if (!f || cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
+            return 0;
+        if (smem > (size_t)dev_smem) return 0;
+        if (threads) *threads = th;
+        if (fn) *fn = f;
+        return smem;
+    }
+
+    // U contour steps of nchain chains, one launch per phase; segments < NsA take w[0], the rest
+    // w[1]; x: exchange buffers, one field per chain and layout ([chain], [2 + chain])
+    int contour_steps(int nchain, const ChainSpan* ch, const double* const w[2], long long NsA, size_t U, double* const* x,
+                      cudaStream_t st) {
+        int threads = 0, grid = 1;
+        ContourStepFn f = nullptr;
+        const size_t smem = step_smem(&threads, &f);
+        CKR(grant_pass((const void*)f, threads, smem, &grid));
+        const int n = (int)grid_phy[0];
+        grid = std::min(grid, nchain * n);
+        auto factor = [&](const ChainSpan& c, long long step) {
+            const long long slot = c.slot0 + c.dir * step;
+            return w[(c.dir > 0 ? slot : slot - 1) < NsA ? 0 : 1];
+        };
+        for (long long k = 0; k <= (long long)U; ++k) {
+            ContourStepArgs a{};
+            a.plane = (k & 1) == 0;
+            a.nchain = nchain;
+            a.finish = k >= 1;
+            a.start = k < (long long)U;
+            a.opz = ops->d_mma.p + ops->mma[2].off;
+            a.opc = ops->d_mma.p + ops->mma[a.plane ? 1 : 0].off;
+            for (int c = 0; c < nchain; ++c) {
+                double* slice = ch[c].q + (ch[c].slot0 + ch[c].dir * k) * (long long)M;
+                a.in[c] = k == 0 ? slice : x[(a.plane ? 2 : 0) + c];
+                a.q[c] = slice;
+                a.xout[c] = x[(a.plane ? 0 : 2) + c];
+                if (a.finish) a.w0[c] = factor(ch[c], k - 1);
+                if (a.start) a.w1[c] = factor(ch[c], k);
+            }
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)grid);
+            cfg.blockDim = dim3((unsigned)threads);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            CK(cudaLaunchKernelEx(&cfg, f, a));
+            ++launches;
+        }
+        return SCFT_OK;
+    }
+
+    // whether the FP32 tensor-core axis passes (axis_dmma.cuh, 3xTF32) run this grid by default,
+    // on a cubic grid with a side the kernels cover (96 or 128), from measurements on one B200:
+    // PMMM always; P1 for both chains of an iteration (128^3: 69.7 against 62.1 iterations/s) but
+    // not for one chain; never 3m (52.8 against 44.2 iterations/s by FFT at 256^3)
+    bool tf32_axis_passes(int nchain) const {
+        const OpsSet* o = ops;
+        if (kind == SCFT_SOLVER_3M || (kind == SCFT_SOLVER_P1 && nchain < 2)) return false;
+        if (o->nterms != 1 || grid_phy[1] != grid_phy[0] || grid_phy[2] != grid_phy[0]) return false;
+        if (o->eo_f32[0] != o->eo_f32[1] || o->eo_f32[1] != o->eo_f32[2]) return false;
+        size_t smem = 0, stride = 0;
+        return axis_tf32_kernel_for((int)grid_phy[0], o->eo_f32[0], 2, &smem, &stride) != nullptr;
+    }
+
+    template <typename T>
+    AxisFftFn<T> fft_kernel(int ax, size_t* smem) const {
+        if (!ops->fft_nf[ax]) return nullptr;
+        return axis_fft_kernel_for<T>((int)grid_phy[ax], ops->fft_nf[ax], ops->fft_ext[ax], smem);
+    }
+
+    // one FFT pass (axis_fft.cuh) along axis ax; pre and post on the z and x pass as in the others
+    template <typename T>
+    int fft_pass(int ax, int nchain, const T* const in[2], T* const out[2], const T* const pre[2],
+                 const T* const post[2], cudaStream_t st) {
+        const OpsSet* o = ops;
+        size_t smem = 0;
+        const AxisFftFn<T> f = fft_kernel<T>(ax, &smem);
+        AxisFftPass<T> p{};
+        for (int c = 0; c < nchain; ++c) {
+            p.in[c] = in[c];
+            p.out[c] = out[c];
+            p.pre[c] = pre ? pre[c] : nullptr;
+            p.post[c] = post ? post[c] : nullptr;
+        }
+        p.nchain = nchain;
+        if constexpr (sizeof(T) == 8) {
+            p.tw = o->d_fft_tw[ax].p;
+            p.g = o->d_fft_g[ax].p;
+        } else {
+            p.tw = o->f_fft_tw[ax].p;
+            p.g = o->f_fft_g[ax].p;
+        }
+        const long long nx = (long long)grid_phy[0], ny = (long long)grid_phy[1], nz = (long long)grid_phy[2];
+        p.outer = ax == 2 ? nx * ny : (ax == 1 ? nx : 1);
+        p.inner = ax == 2 ? 1 : (ax == 1 ? nz : ny * nz);
+        int grid = 1;
+        CKR(grant_pass((const void*)f, kFftThreads, smem, &grid));
+        f<<<grid, kFftThreads, smem, st>>>(p);
+        CK(cudaGetLastError());
+        ++launches;
+        return SCFT_OK;
+    }
+
+    // the three passes of an FP32 triplet by FFT; *done = false if an axis has no FFT form or the
+    // dense form is to run
+    int triplet_fft_f32(int nchain, const ChainIO<float> io[2], float* t1[2], float* t2[2], cudaStream_t st, bool* done) {
+        *done = false;
+        if (ops->nterms != 1) return SCFT_OK;
         const int form = axis_form_override();
         if (form == 2) return SCFT_OK;
-        if (form == 0 && tensor_axis_passes<T>(nchain)) return SCFT_OK;  // measured faster there
-        AxisFftFn<T> f[3];
-        size_t sm[3];
+        if (form == 0 && tf32_axis_passes(nchain)) return SCFT_OK;  // measured faster there
         for (int ax = 0; ax < 3; ++ax) {
-            if (!o->fft_nf[ax]) return SCFT_OK;
-            f[ax] = axis_fft_kernel_for<T>((int)grid_phy[ax], o->fft_nf[ax], o->fft_ext[ax], &sm[ax]);
-            if (!f[ax]) return SCFT_OK;
+            size_t smem = 0;
+            if (!fft_kernel<float>(ax, &smem)) return SCFT_OK;
         }
-        if (!sms) CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        const int nx = (int)grid_phy[0], ny = (int)grid_phy[1], nz = (int)grid_phy[2];
-        for (int ax = 2; ax >= 0; --ax) {
-            bool set = false;
-            for (const void* p : fft_fn_set) set |= p == (const void*)f[ax];
-            if (!set) {
-                CK(cudaFuncSetAttribute(f[ax], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm[ax]));
-                fft_fn_set.push_back((const void*)f[ax]);
-            }
-            AxisFftPass<T> p{};
-            for (int c = 0; c < nchain; ++c) {
-                p.in[c] = ax == 2 ? io[c].in : (ax == 1 ? t1[c] : t2[c]);
-                p.out[c] = ax == 2 ? t1[c] : (ax == 1 ? t2[c] : io[c].out);
-                p.pre[c] = ax == 2 ? io[c].pre : nullptr;
-                p.post[c] = ax == 0 ? io[c].post : nullptr;
-            }
-            p.nchain = nchain;
-            if constexpr (sizeof(T) == 8) {
-                p.tw = o->d_fft_tw[ax].p;
-                p.g = o->d_fft_g[ax].p;
-            } else {
-                p.tw = o->f_fft_tw[ax].p;
-                p.g = o->f_fft_g[ax].p;
-            }
-            p.outer = ax == 2 ? (long long)nx * ny : (ax == 1 ? nx : 1);
-            p.inner = ax == 2 ? 1 : (ax == 1 ? nz : (long long)ny * nz);
-            int per_sm = 1;
-            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f[ax], kFftThreads, sm[ax]));
-            f[ax]<<<sms * (per_sm > 0 ? per_sm : 1), kFftThreads, sm[ax], st>>>(p);
-            CK(cudaGetLastError());
-        }
-        launches += 3;
+        const float* in[2] = {io[0].in, io[1].in};
+        float* out[2] = {io[0].out, io[1].out};
+        const float* pre[2] = {io[0].pre, io[1].pre};
+        const float* post[2] = {io[0].post, io[1].post};
+        const float* c1[2] = {t1[0], t1[1]};
+        const float* c2[2] = {t2[0], t2[1]};
+        CKR(fft_pass<float>(2, nchain, in, t1, pre, nullptr, st));
+        CKR(fft_pass<float>(1, nchain, c1, t2, nullptr, nullptr, st));
+        CKR(fft_pass<float>(0, nchain, c2, out, nullptr, post, st));
         *done = true;
+        return SCFT_OK;
+    }
+
+    // one SIMT pass (axis_kernels.cuh) along axis ax of term o
+    template <typename T>
+    int simt_pass(int ax, OpsSet* o, int nchain, const T* const in[2], T* const out[2], const T* const pre[2],
+                  const T* const post[2], bool accum, cudaStream_t st) {
+        const int nx = (int)grid_phy[0], ny = (int)grid_phy[1], nz = (int)grid_phy[2];
+        AxisPass<T> p{};
+        for (int c = 0; c < nchain; ++c)
+            p.ch[c] = ChainIO<T>{in[c], out[c], pre ? pre[c] : nullptr, post ? post[c] : nullptr, accum};
+        if constexpr (sizeof(T) == 8) {
+            p.op = o->d_op[ax].p;
+            p.opT = o->d_opT[ax].p;
+        } else {
+            p.op = o->f_op[ax].p;
+            p.opT = o->f_opT[ax].p;
+        }
+        p.n = (int)grid_phy[ax];
+        p.outer = ax == 2 ? (long long)nx * ny : (ax == 1 ? nx : 1);
+        p.inner = ax == 2 ? 1 : (ax == 1 ? nz : (long long)ny * nz);
+        CK(launch_axis(p, nchain, ax == 2, st));
+        ++launches;
         return SCFT_OK;
     }
 
@@ -762,6 +1041,12 @@ struct scft_solver_s {
         s->nterms = nt;
         for (int t = 1; t < nt; ++t) s->more.push_back(std::make_unique<OpsSet>());
         int eo2_axes = 0;
+        std::vector<std::vector<double>> h_mma((size_t)nt);
+        // 3m without translations is PMMM in another order of the points
+        const bool m3_plain = kind == SCFT_SOLVER_3M && nt == 1 && m3sym.par[0] == 0 && m3sym.par[1] == 0 &&
+                              m3sym.par[2] == 0 && m3_no_half_cells();
+        s->pos_order = m3_plain && grid_phy[0] <= (size_t)kMmaMaxN && grid_phy[1] <= (size_t)kMmaMaxN &&
+                       grid_phy[2] <= (size_t)kMmaMaxN;
         for (int ax = 0; ax < 3; ++ax) {
             std::vector<long double> A;
             const int N = (int)grid_log[ax];
@@ -771,20 +1056,22 @@ struct scft_solver_s {
                 A = p1_axis_operator(N, (long double)cell[ax], (long double)ds_);
             } else {
                 const std::vector<long double> c = circulant_kernel(N, (long double)cell[ax], (long double)ds_);
-                for (int t = 1; t < nt; ++t)
-                    CKR(upload_operator(m3_axis_factor(c, N, m3sym.par[ax], m3terms[(size_t)t][ax]),
-                                        (int)grid_phy[ax], *s->term(t), ax));
+                for (int t = 1; t < nt; ++t) {
+                    const std::vector<long double> B = m3_axis_factor(c, N, m3sym.par[ax], m3terms[(size_t)t][ax]);
+                    CKR(upload_operator(B, (int)grid_phy[ax], *s->term(t), ax));
+                    OpsSet* o = s->term(t);
+                    pack_operator_mma(B, (int)grid_phy[ax], false, o->mma[ax], h_mma[(size_t)t], OpsSet::before(o->mma, ax));
+                }
                 A = m3_axis_factor(c, N, m3sym.par[ax], m3terms[0][ax]);
             }
             CKR(upload_operator(A, (int)grid_phy[ax], *s, ax));
-            pack_operator(A, (int)grid_phy[ax], *s, ax);
+            pack_operator_mma(A, (int)grid_phy[ax], m3_plain, s->mma[ax], h_mma[0], OpsSet::before(s->mma, ax));
+            pack_operator(s->pos_order ? position_order(A, (int)grid_phy[ax]) : A, (int)grid_phy[ax], *s, ax);
             pack_operator_f32(A, (int)grid_phy[ax], *s, ax);
             if (nt == 1 && s->h16_axes == ax) pack_operator_h16(A, (int)grid_phy[ax], *s);
             {
                 const int n = (int)grid_phy[ax];
                 int nf = 0, ext = 0;
-                const bool m3_plain = kind == SCFT_SOLVER_3M && nt == 1 && m3sym.par[0] == 0 && m3sym.par[1] == 0 &&
-                                      m3sym.par[2] == 0 && m3_no_half_cells();
                 if (kind == SCFT_SOLVER_P1) nf = n;
                 else if (kind == SCFT_SOLVER_PMMM) { nf = 2 * n; ext = 1; }
                 else if (m3_plain) { nf = 2 * n; ext = 2; }
@@ -792,7 +1079,13 @@ struct scft_solver_s {
                 if (nf && axis_fft_kernel_for<double>(n, nf, ext, &fsm))
                     CKR(upload_fft_tables(*s, ax, nf, ext, (long double)cell[ax], (long double)ds_));
             }
-            eo2_axes += (kind == SCFT_SOLVER_PMMM && nt == 1 && pack_operator_eo2(A, (int)grid_phy[ax], *s)) ? 1 : 0;
+            if (kind == SCFT_SOLVER_PMMM && nt == 1) eo2_axes += pack_operator_eo2(A, (int)grid_phy[ax], *s) ? 1 : 0;
+            else if (s->pos_order)
+                eo2_axes += pack_operator_eo2(position_order(A, (int)grid_phy[ax]), (int)grid_phy[ax], *s) ? 1 : 0;
+        }
+        for (int t = 0; t < nt; ++t) {
+            CKR(s->term(t)->d_mma.alloc(h_mma[(size_t)t].size()));
+            CKR(upload(s->term(t)->d_mma.p, h_mma[(size_t)t].data(), h_mma[(size_t)t].size() * sizeof(double)));
         }
         s->eo2 = eo2_axes == 3;
         if (s->eo2) {
@@ -817,6 +1110,7 @@ struct scft_solver_s {
     int build_dops() {
         if (!ops) return fail(SCFT_ERR_NOT_READY, "set_cell_para/set_contour_step first");
         if (ops->have_dop) return SCFT_OK;
+        std::vector<std::vector<double>> h_mma((size_t)ops->nterms);
         for (int ax = 0; ax < 3; ++ax) {
             const int N = (int)grid_log[ax];
             const int n = (int)grid_phy[ax];
@@ -837,93 +1131,66 @@ struct scft_solver_s {
                         dt[(size_t)j * n + i] = (double)A[(size_t)i * n + j];
                     }
                 OpsSet* o = ops->term(t);
+                // the derivative keeps the operator's symmetry, and so its point order
+                pack_operator_mma(A, n, o->mma[ax].perm != 0, o->dmma[ax], h_mma[(size_t)t], OpsSet::before(o->dmma, ax));
                 CKR(o->d_dop[ax].alloc((size_t)n * n));
                 CKR(o->d_dopT[ax].alloc((size_t)n * n));
                 CKR(upload(o->d_dop[ax].p, d.data(), d.size() * sizeof(double)));
                 CKR(upload(o->d_dopT[ax].p, dt.data(), dt.size() * sizeof(double)));
             }
         }
+        for (int t = 0; t < ops->nterms; ++t) {
+            OpsSet* o = ops->term(t);
+            CKR(o->d_dmma.alloc(h_mma[(size_t)t].size()));
+            CKR(upload(o->d_dmma.p, h_mma[(size_t)t].data(), h_mma[(size_t)t].size() * sizeof(double)));
+        }
         ops->have_dop = true;
         return SCFT_OK;
     }
 
-    // (op_x (x) op_y (x) op_z) applied to nt stacked fields: in -> t1 -> t2 -> out
-    int triplet_batched(const double* in, double* out, double* t1, double* t2, long long nt,
-                        const double* const op[3], const double* const opT[3], cudaStream_t st) {
-        const int nx = (int)grid_phy[0], ny = (int)grid_phy[1], nz = (int)grid_phy[2];
-        AxisPass<double> pz{}, py{}, px{};
-        pz.ch[0] = ChainIO<double>{in, t1, nullptr, nullptr};
-        py.ch[0] = ChainIO<double>{t1, t2, nullptr, nullptr};
-        px.ch[0] = ChainIO<double>{t2, out, nullptr, nullptr};
-        pz.op = op[2]; pz.opT = opT[2]; pz.n = nz; pz.outer = nt * nx * ny; pz.inner = 1;
-        py.op = op[1]; py.opT = opT[1]; py.n = ny; py.outer = nt * nx; py.inner = nz;
-        px.op = op[0]; px.opT = opT[0]; px.n = nx; px.outer = nt; px.inner = (long long)ny * nz;
-        CK(launch_axis(pz, 1, true, st));
-        CK(launch_axis(py, 1, false, st));
-        CK(launch_axis(px, 1, false, st));
+    // the derivative triplet by L_dax (axis dax's operator replaced by its derivative) of term o,
+    // applied to nt stacked fields: in -> t1 -> t2 -> out
+    int triplet_batched(const double* in, double* out, double* t1, double* t2, long long nt, OpsSet* o, int dax,
+                        cudaStream_t st, bool in_positions) {
+        const double* src[3] = {t2, t1, in};
+        double* dst[3] = {out, t2, t1};
+        for (int ax = 2; ax >= 0; --ax) {
+            const OpsSet::Mma& m = ax == dax ? o->dmma[ax] : o->mma[ax];
+            if (m.mode >= 0) {
+                const double* i2[2] = {src[ax], nullptr};
+                double* o2[2] = {dst[ax], nullptr};
+                CKR(mma_pass(ax, m, ax == dax ? o->d_dmma.p : o->d_mma.p, 1, i2, o2, nullptr, nullptr, nt, false, false, st,
+                             in_positions));
+                continue;
+            }
+            const long long nx = (long long)grid_phy[0], ny = (long long)grid_phy[1], nz = (long long)grid_phy[2];
+            AxisPass<double> p{};
+            p.ch[0] = ChainIO<double>{src[ax], dst[ax], nullptr, nullptr};
+            p.op = ax == dax ? o->d_dop[ax].p : o->d_op[ax].p;
+            p.opT = ax == dax ? o->d_dopT[ax].p : o->d_opT[ax].p;
+            p.n = (int)grid_phy[ax];
+            p.outer = nt * (ax == 2 ? nx * ny : (ax == 1 ? nx : 1));
+            p.inner = ax == 2 ? 1 : (ax == 1 ? nz : ny * nz);
+            CK(launch_axis(p, 1, ax == 2, st));
+        }
         return SCFT_OK;
     }
 
     // one triplet per chain: in -> (pre) z-pass -> t1 -> y-pass -> t2 -> x-pass (post) -> out
     // A multi-term operator (ops->nterms > 1) runs the three passes per term and adds the
     // x passes up in `out`, so there `in` and `out` must not alias.
+    // in_positions: the FP64 fields are in position order (pos_order operators).
     template <typename T>
-    int triplet(int nchain, const ChainIO<T> io[2], T* t1[2], T* t2[2], cudaStream_t st) {
+    int triplet(int nchain, const ChainIO<T> io[2], T* t1[2], T* t2[2], cudaStream_t st, bool in_positions = false) {
         const int nx = (int)grid_phy[0], ny = (int)grid_phy[1], nz = (int)grid_phy[2];
         const int nt = ops->nterms;
         for (int c = 0; c < nchain && nt > 1; ++c)
             if ((const void*)io[c].in == (const void*)io[c].out)
                 return fail(SCFT_ERR_INVALID_ARG, "multi-term triplet: input and output alias");
-        {
+        if constexpr (sizeof(T) == 4) {
             bool done = false;
-            CKR(triplet_fft<T>(nchain, io, t1, t2, st, &done));
+            CKR(triplet_fft_f32(nchain, io, t1, t2, st, &done));
             if (done) return SCFT_OK;
-        }
-        if constexpr (sizeof(T) == 8) {
-            // large cubic grids: the three passes on the FP64 tensor cores (axis_dmma.cuh)
-            if (nt == 1 && nx == ny && ny == nz && ops->eo[0] == ops->eo[1] && ops->eo[1] == ops->eo[2]) {
-                AxisDmmaFn f[3];
-                size_t smem = 0;
-                const bool eo2 = ops->eo2 && nx == 128;
-                for (int ax = 0; ax < 3; ++ax) f[ax] = axis_dmma_kernel_for(nx, ops->eo[ax], ax, &smem, eo2);
-                if (f[0] && f[1] && f[2]) {
-                    if (!sms) CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-                    if (axis_dmma_smem_set != smem || axis_dmma_fn_set != (const void*)f[2]) {
-                        for (int ax = 0; ax < 3; ++ax)
-                            CK(cudaFuncSetAttribute(f[ax], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-                        axis_dmma_smem_set = smem;
-                        axis_dmma_fn_set = (const void*)f[2];
-                    }
-                    AxisPassD pz{}, py{}, px{};
-                    for (int c = 0; c < nchain; ++c) {
-                        pz.in[c] = io[c].in; pz.out[c] = t1[c]; pz.pre[c] = io[c].pre;
-                        py.in[c] = t1[c]; py.out[c] = t2[c];
-                        px.in[c] = t2[c]; px.out[c] = io[c].out; px.post[c] = io[c].post;
-                    }
-                    pz.nchain = py.nchain = px.nchain = nchain;
-                    pz.hints = py.hints = px.hints = l2_hints_enabled();
-                    py.discard_in = px.discard_in = l2_hints_enabled();  // t1, t2: dead once read
-                    if (eo2) {
-                        const size_t per_axis = ops->h_packed2.size() / 3;  // AxisShapeEO2<n>::SIZE
-                        pz.op = ops->d_packed2.p + 2 * per_axis;
-                        py.op = ops->d_packed2.p + per_axis;
-                        px.op = ops->d_packed2.p;
-                    } else {
-                        pz.op = ops->d_packed.p + ops->off[2];
-                        py.op = ops->d_packed.p + ops->off[1];
-                        px.op = ops->d_packed.p + ops->off[0];
-                    }
-                    f[2]<<<sms, kContourThreads, smem, st>>>(pz);
-                    CK(cudaGetLastError());
-                    f[1]<<<sms, kContourThreads, smem, st>>>(py);
-                    CK(cudaGetLastError());
-                    f[0]<<<sms, kContourThreads, smem, st>>>(px);
-                    CK(cudaGetLastError());
-                    launches += 3;
-                    return SCFT_OK;
-                }
-            }
-        } else {
             // large cubic grids, FP32 precision form: 3xTF32 axis passes
             if (nt == 1 && nx == ny && ny == nz && ops->eo_f32[0] == ops->eo_f32[1] &&
                 ops->eo_f32[1] == ops->eo_f32[2]) {
@@ -964,34 +1231,38 @@ struct scft_solver_s {
                 }
             }
         }
+        const T* src[2] = {io[0].in, io[1].in};
+        T* dst[2] = {io[0].out, io[1].out};
+        const T* pre[2] = {io[0].pre, io[1].pre};
+        const T* post[2] = {io[0].post, io[1].post};
+        const T* c1[2] = {t1[0], t1[1]};
+        const T* c2[2] = {t2[0], t2[1]};
         for (int t = 0; t < nt; ++t) {
             OpsSet* o = ops->term(t);
-            const T* opx;
-            const T* opy;
-            const T* opz;
-            const T* opxT;
-            const T* opyT;
-            const T* opzT;
-            if constexpr (sizeof(T) == 8) {
-                opx = (const T*)o->d_op[0].p; opy = (const T*)o->d_op[1].p; opz = (const T*)o->d_op[2].p;
-                opxT = (const T*)o->d_opT[0].p; opyT = (const T*)o->d_opT[1].p; opzT = (const T*)o->d_opT[2].p;
-            } else {
-                opx = (const T*)o->f_op[0].p; opy = (const T*)o->f_op[1].p; opz = (const T*)o->f_op[2].p;
-                opxT = (const T*)o->f_opT[0].p; opyT = (const T*)o->f_opT[1].p; opzT = (const T*)o->f_opT[2].p;
+            for (int ax = 2; ax >= 0; --ax) {
+                const T* const* in = ax == 2 ? src : (ax == 1 ? c1 : c2);
+                T* const* out = ax == 2 ? t1 : (ax == 1 ? t2 : dst);
+                const T* const* pr = ax == 2 ? pre : nullptr;
+                const T* const* po = ax == 0 && t == nt - 1 ? post : nullptr;
+                const bool accum = ax == 0 && t > 0;
+                if constexpr (sizeof(T) == 8) {
+                    // the tensor-core pass up to kMmaMaxN points, the FFT beyond (256-point axes)
+                    const int form = nt == 1 ? axis_form_override() : 2;
+                    size_t smem = 0;
+                    const bool fft = nt == 1 && !in_positions && fft_kernel<T>(ax, &smem) != nullptr;
+                    if (o->mma[ax].mode >= 0 && !(form == 1 && fft)) {
+                        // t1 and t2 are dead once read
+                        CKR(mma_pass(ax, o->mma[ax], o->d_mma.p, nchain, in, out, pr, po, 1, accum,
+                                     ax != 2 && l2_hints_enabled(), st, in_positions));
+                        continue;
+                    }
+                    if (fft && form != 2) {
+                        CKR(fft_pass<T>(ax, nchain, in, out, pr, po, st));
+                        continue;
+                    }
+                }
+                CKR(simt_pass<T>(ax, o, nchain, in, out, pr, po, accum, st));
             }
-            AxisPass<T> pz{}, py{}, px{};
-            for (int c = 0; c < nchain; ++c) {
-                pz.ch[c] = ChainIO<T>{io[c].in, t1[c], io[c].pre, nullptr};
-                py.ch[c] = ChainIO<T>{t1[c], t2[c], nullptr, nullptr};
-                px.ch[c] = ChainIO<T>{t2[c], io[c].out, nullptr, t == nt - 1 ? io[c].post : nullptr, t > 0};
-            }
-            pz.op = opz; pz.opT = opzT; pz.n = nz; pz.outer = (long long)nx * ny; pz.inner = 1;
-            py.op = opy; py.opT = opyT; py.n = ny; py.outer = nx; py.inner = nz;
-            px.op = opx; px.opT = opxT; px.n = nx; px.outer = 1; px.inner = (long long)ny * nz;
-            CK(launch_axis(pz, nchain, true, st));
-            CK(launch_axis(py, nchain, false, st));
-            CK(launch_axis(px, nchain, false, st));
-            launches += 3;
         }
         return SCFT_OK;
     }
@@ -1048,11 +1319,24 @@ struct scft_diblock_s {
     unsigned long long saved_gen[2] = {~0ULL, ~0ULL};
     bool saved_use_graph[2] = {true, true};
 
+    // second stream of an iteration whose chains are launched step by step
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_fork = nullptr, side_join = nullptr;
+    int make_side() {
+        if (!side) CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        if (!side_fork) CK(cudaEventCreateWithFlags(&side_fork, cudaEventDisableTiming));
+        if (!side_join) CK(cudaEventCreateWithFlags(&side_join, cudaEventDisableTiming));
+        return SCFT_OK;
+    }
+
     // page-locked staging of the end-to-end form: hist_cap history rows, then the error word
     double* pin_out = nullptr;
 
     ~scft_diblock_s() {
         if (pin_out) cudaFreeHost(pin_out);
+        if (side_fork) cudaEventDestroy(side_fork);
+        if (side_join) cudaEventDestroy(side_join);
+        if (side) cudaStreamDestroy(side);
         if (gexec) cudaGraphExecDestroy(gexec);
         if (graph) cudaGraphDestroy(graph);
         for (int i = 0; i < 2; ++i) {
@@ -1349,8 +1633,15 @@ struct scft_diblock_s {
         const int blocks = grid_blocks(MM, 256);
         size_t launches = 0;
         bool fused = false;  // phi was summed by this iteration's contour kernel
+        PointOrder po{};
+        if (sizeof(T) == 8 && solver->ops->pos_order) {
+            po.on = 1;
+            po.nx = (int)solver->grid_phy[0];
+            po.ny = (int)solver->grid_phy[1];
+            po.nz = (int)solver->grid_phy[2];
+        }
         if (parts & kPartPrep) {
-            prep_kernel<T><<<blocks, 256, 0, st>>>(wA.p, wB.p, ksi.p, wAds, wBds, q, qc + U * M, xN, ds, MM);
+            prep_kernel<T><<<blocks, 256, 0, st>>>(wA.p, wB.p, ksi.p, wAds, wBds, q, qc + U * M, xN, ds, MM, po);
             CK(cudaGetLastError());
             ++launches;
         }
@@ -1367,7 +1658,27 @@ struct scft_diblock_s {
                 }
                 ++solver->launches;
             }
-            for (size_t t_ = 0; t_ < U && !persistent; ++t_) {
+            bool stepped = false;
+            if constexpr (sizeof(T) == 8) {
+                if (!persistent && solver->step_smem()) {
+                    // each chain on a stream of its own: the launches of one chain fill the SMs that
+                    // the other's leave (2 x 128 planes on 148 SMs are 1.73 rounds, not 2), and one
+                    // chain's loads and stores run under the other's MMAs
+                    const ChainSpan ch[2] = {{q, 0, 1}, {qc, (long long)U, -1}};
+                    const double* w[2] = {wAds, wBds};
+                    double* x0[4] = {t[0], nullptr, t[2], nullptr};
+                    double* x1[4] = {t[1], nullptr, t[3], nullptr};
+                    CKR(make_side());
+                    CK(cudaEventRecord(side_fork, st));
+                    CK(cudaStreamWaitEvent(side, side_fork, 0));
+                    CKR(solver->contour_steps(1, &ch[0], w, (long long)NsA, U, x0, st));
+                    CKR(solver->contour_steps(1, &ch[1], w, (long long)NsA, U, x1, side));
+                    CK(cudaEventRecord(side_join, side));
+                    CK(cudaStreamWaitEvent(st, side_join, 0));
+                    stepped = true;
+                }
+            }
+            for (size_t t_ = 0; t_ < U && !persistent && !stepped; ++t_) {
                 // forward chain: q[t] -> q[t+1] with block A (t < NsA) or B
                 // backward chain: qc[U-t] -> qc[U-t-1] with the block of segment U-t-1
                 const T* w1 = t_ < NsA ? wAds : wBds;
@@ -1378,7 +1689,7 @@ struct scft_diblock_s {
                 io[1] = ChainIO<T>{qc + (ub + 1) * M, qc + ub * M, w2, w2};
                 T* t1[2] = {t[0], t[1]};
                 T* t2[2] = {t[2], t[3]};
-                CKR(solver->triplet<T>(2, io, t1, t2, st));
+                CKR(solver->triplet<T>(2, io, t1, t2, st, po.on != 0));
             }
             launches += solver->launches - before;
             if (phase_events) CK(cudaEventRecord(phase_events[2], st));
@@ -1393,10 +1704,10 @@ struct scft_diblock_s {
         if (fused)
             phi_fused_finish_kernel<T><<<grid_blocks(MM, 256), 256, 0, st>>>(
                 phi_acc.p, q, qc, phiA.p, phiB.p, state.p, fA, (long long)NsA, (long long)NsB,
-                (int)solver->grid_phy[0]);
+                (int)solver->grid_phy[0], po);
         else
             phi_kernel<T><<<grid_blocks((MM + 1) / 2, 256), 256, 0, st>>>(q, qc, phiA.p, phiB.p, state.p, fA,
-                                                                          (long long)NsA, (long long)NsB, MM);
+                                                                          (long long)NsA, (long long)NsB, MM, po);
         CK(cudaGetLastError());
         if (phase_events) CK(cudaEventRecord(phase_events[3], st));
         energy_kernel<<<rblocks, kRedThreads, 0, st>>>(wA.p, wB.p, phiA.p, phiB.p, ksi.p, xN, MM,
@@ -1726,6 +2037,15 @@ int scft_solver_propagate_device(scft_solver_t s, double* d_q, const double* d_i
     const size_t M = s->M;
     size_t slot = direction == 1 ? 0 : Ns;
     CK(cudaMemcpyAsync(d_q + slot * M, d_init, M * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    // one launch per step where the step kernel covers the grid; it moves 16-byte words, so the
+    // caller's arrays must be aligned to them (the three passes take any)
+    const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    if (Ns > 0 && !s->ops->mma[0].perm && aligned(d_q) && aligned(d_wds) && s->step_smem()) {
+        const ChainSpan ch{d_q, (long long)slot, direction};
+        const double* w[2] = {d_wds, d_wds};
+        double* x[4] = {s->d_t1.p, nullptr, s->d_t2.p, nullptr};
+        return s->contour_steps(1, &ch, w, 0, Ns, x, st);
+    }
     for (size_t k = 0; k < Ns; ++k) {
         const size_t next = direction == 1 ? slot + 1 : slot - 1;
         ChainIO<double> io[2] = {{d_q + slot * M, d_q + next * M, d_wds, d_wds}, {}};
@@ -1989,13 +2309,7 @@ int scft_diblock_stress(scft_diblock_t d, double dlnQ_dL[3], double* dF_dxN, dou
       // d/dL_a of a sum of Kronecker products: the sum over terms of each term with its
       // axis-a factor replaced by the derivative factor
       for (int term = 0; term < s->ops->nterms; ++term) {
-        const OpsSet* o = s->ops->term(term);
-        const double* op[3];
-        const double* opT[3];
-        for (int b = 0; b < 3; ++b) {
-            op[b] = b == ax ? o->d_dop[b].p : o->d_op[b].p;
-            opT[b] = b == ax ? o->d_dopT[b].p : o->d_opT[b].p;
-        }
+        OpsSet* o = s->ops->term(term);
         for (int blk = 0; blk < 2; ++blk) {
             const long long lo = blk == 0 ? 0 : NsA, hi = blk == 0 ? NsA : U;
             const double* D = blk == 0 ? d->d_wAds.p : d->d_wBds.p;
@@ -2007,7 +2321,7 @@ int scft_diblock_stress(scft_diblock_t d, double dlnQ_dL[3], double* dF_dxN, dou
                 else
                     stress_scale_kernel<double><<<grid_blocks(nt * M, 256), 256, 0, st>>>(X, d->d_q.p, D, t0, nt, M);
                 CK(cudaGetLastError());
-                CKR(s->triplet_batched(X, Y, T1, T2, nt, op, opT, st));
+                CKR(s->triplet_batched(X, Y, T1, T2, nt, o, ax, st, !f32 && s->ops->pos_order));
                 const int nb = (int)std::min<long long>(rblocks, (nt * M + kRedThreads - 1) / kRedThreads);
                 if (f32)
                     stress_dot_kernel<float><<<nb, kRedThreads, 0, st>>>(d->f_qc.p, Df, Y, t0, nt, M, d->partials.p);
@@ -2051,8 +2365,18 @@ int scft_diblock_get_contour(scft_diblock_t d, int chain, size_t slot, double* o
     const size_t M = d->M;
     if (d->precision == SCFT_FP64) {
         const double* src = (chain ? d->d_qc.p : d->d_q.p) + slot * M;
-        CK(cudaMemcpyAsync(out, src, M * sizeof(double), cudaMemcpyDeviceToHost, st));
+        const bool pos = d->solver->ops && d->solver->ops->pos_order;
+        std::vector<double> tmp(pos ? M : 0);
+        CK(cudaMemcpyAsync(pos ? tmp.data() : out, src, M * sizeof(double), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if (pos) {  // the store is in position order
+            const size_t* g = d->solver->grid_phy;
+            auto at = [](size_t j, size_t n) { return (j & 1) ? n - 1 - (j >> 1) : (j >> 1); };
+            for (size_t x = 0, i = 0; x < g[0]; ++x)
+                for (size_t y = 0; y < g[1]; ++y)
+                    for (size_t z = 0; z < g[2]; ++z, ++i)
+                        out[(at(x, g[0]) * g[1] + at(y, g[1])) * g[2] + at(z, g[2])] = tmp[i];
+        }
     } else {
         std::vector<float> tmp(M);
         const float* src = (chain ? d->f_qc.p : d->f_q.p) + slot * M;

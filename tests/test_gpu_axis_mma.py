@@ -1,0 +1,110 @@
+"""FP64 tensor-core axis passes and the one-launch-per-step kernel at the edges of their tiles:
+triplets and chains against the dense per-axis operators, iterations against the numpy oracle."""
+import numpy as np
+import pytest
+
+from crysscft_sample_b200 import fields, scft, solvers
+from oracle import scft_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+L = (4.2, 3.9, 5.1)
+U64 = 2.0**-53
+
+
+def _solver(kind, N, cell=None, ds=0.01):
+    G = solvers.make_solver(kind, N)
+    G.set_cell_para(cell if cell is not None else ((L[0],) * 3 if kind == "PMMM" else L))
+    G.set_contour_step(ds)
+    return G
+
+
+def _operators(kind, N, cell=None, ds=0.01):
+    cell = cell if cell is not None else ((L[0],) * 3 if kind == "PMMM" else L)
+    return solvers.operator_terms(kind, N, cell, ds)[0]
+
+
+def _apply(A, q):
+    q = np.einsum("xyj,zj->xyz", q, A[2])
+    q = np.einsum("xjz,yj->xyz", q, A[1])
+    return np.einsum("jyz,xj->xyz", q, A[0])
+
+
+def _bound(n, q):
+    # dot products of n terms on each axis: gamma_n with row sums of |A| below 1.3, twice for the
+    # sums and differences of mirrored points, on both sides of the comparison
+    return 2 * 2 * 1.3**3 * sum(n) * U64 * np.abs(q).max()
+
+
+# lengths around the 8-wide tiles, the 32-line tiles and the block forms (n % 32), odd, tiny and
+# mixed; 64, 96 and 128 have kernels of their own
+GRIDS = [("P1", n) for n in [(1, 2, 3), (7, 9, 5), (8, 16, 24), (31, 33, 32), (63, 65, 64), (96, 64, 128), (127, 17, 97),
+                             (129, 8, 15), (128, 40, 1)]] + \
+        [(k, n) for k in ("PMMM", "3M") for n in [(2, 4, 6), (14, 18, 10), (62, 66, 64), (128, 192, 30), (90, 256, 34)]]
+
+
+@pytest.mark.parametrize("kind,N", GRIDS)
+def test_triplet_equals_dense_operators(gpu, kind, N):
+    G = _solver(kind, N)
+    n = G.get_grid_size_phy()
+    q = np.random.default_rng(1).standard_normal(n)
+    G.get_iomat_for_diffusion()[:] = q.ravel()
+    G.diffusion()
+    got = G.get_iomat_for_diffusion().reshape(n)
+    assert np.abs(got - _apply(_operators(kind, N), q)).max() <= _bound(n, q)
+
+
+# one launch per step (cubic 64, 96, 128; at 128 only with equal axes for PMMM), both directions,
+# and a 16-byte misaligned store, which takes the three passes
+@pytest.mark.parametrize("kind,n,cell", [("P1", 64, L), ("P1", 96, L), ("P1", 128, L), ("PMMM", 64, None),
+                                         ("PMMM", 96, None), ("PMMM", 128, None), ("3M", 64, L), ("P1", 30, L)])
+@pytest.mark.parametrize("direction,offset", [(1, 0), (-1, 0), (1, 1)])
+def test_chain_equals_dense_operators(gpu, kind, n, cell, direction, offset):
+    import torch
+
+    N = (n, n, n) if kind == "P1" else (2 * n,) * 3
+    G, A, steps = _solver(kind, N, cell), _operators(kind, N, cell), 3
+    rng = np.random.default_rng(2)
+    init, w = 1 + 0.1 * rng.standard_normal((n, n, n)), np.exp(0.01 * rng.standard_normal((n, n, n)))
+    store = torch.zeros((steps + 1) * n**3 + offset, dtype=torch.float64, device="cuda")
+    q = store[offset:]
+    G.propagate_device(q, torch.from_numpy(init).cuda().ravel(), torch.from_numpy(w).cuda().ravel(), steps, direction)
+    torch.cuda.synchronize()
+    got = q.cpu().numpy().reshape(steps + 1, n, n, n)[::direction]
+    want = init
+    for k in range(1, steps + 1):
+        want = w * _apply(A, w * want)
+        assert np.abs(got[k] - want).max() <= k * 1.1 * _bound((n, n, n), want)
+
+
+# iterations on the step kernel (96, 128), the whole-contour kernel in position order (3m, 64) and
+# the passes (ragged, anisotropic), with stress and a stored slice
+@pytest.mark.parametrize("kind,N", [("P1", (96, 96, 96)), ("PMMM", (256, 256, 256)), ("3M", (192, 192, 192)),
+                                    ("3M", (128, 128, 128)), ("3M", (36, 50, 30)), ("P1", (33, 20, 15))])
+def test_iterations_equal_oracle(gpu, kind, N):
+    cell, fA, ds, xN = (4.2, 4.2, 4.2), 0.3, 0.1, 18.0
+    rng = np.random.default_rng(3)
+    if all(v % 2 == 0 for v in N):
+        a, b = (fields.to_physical(kind, w) for w in fields.seed_fields(N, cell[0]))
+    else:
+        a, b = rng.standard_normal(N), rng.standard_normal(N)
+    S = O.OracleSolver(kind, N)
+    want = O.scft_iterations(S, fA, ds, xN, cell, 0.1, 2, a, b)
+    G = solvers.make_solver(kind, N)
+    G.set_cell_para(cell)
+    run = scft.DiblockSCFT(G, fA, ds, xN, 0.1)
+    run.set_fields(a, b)
+    got = run.iterate(2)
+    got.update(run.get_fields())
+    assert np.abs(got["F"] - want["F"]).max() <= 1e-10 * np.abs(want["F"]).max()
+    for k in ("phiA", "phiB"):
+        assert np.abs(got[k] - want[k].ravel()).max() <= 1e-12
+    # a stored slice in the solver's own point order: one step from the one before it
+    S.set_cell_para(cell)
+    S.set_contour_step(ds)
+    run.set_fields(a, b)
+    run.iterate(1)
+    w = np.exp(-ds / 2 * np.asarray(a).ravel())
+    q0, q1 = run.get_contour(0, 1), run.get_contour(0, 2)
+    step = w * np.asarray(S.diffusion((w * q0).reshape(S.grid_phy))).ravel()
+    assert np.abs(q1 - step).max() <= 1e-13 * np.abs(step).max() * 10
