@@ -159,7 +159,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) axis_mma_kernel(const AxisMmaP
             for (int k = 0; k < VPI; ++k) {
                 const long long a = base + (long long)pos(j, k) * inner;
                 v[q * VPI + k] = ok ? __ldcg(in + a) : 0.0;
-                if (ROW) w[ROW ? q * VPI + k : 0] = (ok && pre) ? __ldg(pre + a) : 1.0;
+                if (ROW) w[ROW ? q * VPI + k : 0] = (ok && pre) ? __ldcg(pre + a) : 1.0;
             }
         }
     };
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(kMmaThreads, 2) axis_mma_kernel(const AxisMmaP
                         const long long a = base + (long long)pos(i, k) * inner;
                         double r = y[k];
                         if (p.accum) r = r + out[a];
-                        if (post) r = r * __ldg(post + a);
+                        if (post) r = r * __ldcg(post + a);
                         __stcg(out + a, r);
                     }
                 }

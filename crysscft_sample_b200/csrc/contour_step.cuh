@@ -15,6 +15,11 @@
 // So A_z starts on a warp's rows as soon as its own copies have landed, the finishing and the
 // starting column operation of a phase need no barrier between them, and one barrier (A_z to
 // columns) is left per tile.  The operator blocks are those of axis_mma.cuh (kEo2, kCirc4).
+//
+// 128^3 PMMM, both chains: 53 us a step against 87 us in three passes (256^3 iteration 17.9 -> 11.6
+// ms), P1 43 against 93 us.  DMMA floor 33 us (P1 22); the rest is the 131 KB that a tile moves in
+// and out four times while its SM computes nothing.  16 warps of 8 lines instead of 8 of 16 at 128
+// points: the same time; at 96 points 12 warps.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -184,7 +189,7 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int at = rowpos[k] + (k == 0 || k == 3 ? 8 * r : -8 * r);
-                f[k] = __ldg(reinterpret_cast<const double2*>(w + at * gs + col));
+                f[k] = __ldcg(reinterpret_cast<const double2*>(w + at * gs + col));
             }
         };
         const double* w0 = p.finish ? (c ? p.w0[1] : p.w0[0]) + off : nullptr;
@@ -230,7 +235,7 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
                     const double2 v = make_double2(y0[k] * f[k].x, y1[k] * f[k].y);
                     __stcs(reinterpret_cast<double2*>(q + at * gs + col), v);
                     double2 f1 = f[k];
-                    if (other_w) f1 = __ldg(reinterpret_cast<const double2*>(w1 + at * gs + col));
+                    if (other_w) f1 = __ldcg(reinterpret_cast<const double2*>(w1 + at * gs + col));
                     *reinterpret_cast<double2*>(T + at * LF + col) = make_double2(v.x * f1.x, v.y * f1.y);
                 }
             }
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
             for (int e = lane; e < 8 * ML * (N / 2); e += 32) {
                 const int r = line0 + e / (N / 2), ch = 2 * (e % (N / 2));
                 double2 v = *reinterpret_cast<double2*>(T + r * LF + ch);
-                const double2 f = __ldg(reinterpret_cast<const double2*>(w1 + r * gs + ch));
+                const double2 f = __ldcg(reinterpret_cast<const double2*>(w1 + r * gs + ch));
                 v.x *= f.x;
                 v.y *= f.y;
                 *reinterpret_cast<double2*>(T + r * LF + ch) = v;
@@ -266,6 +271,294 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
                 }
         }
         __syncthreads();  // the columns of T are read: its rows may be fetched again
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same phase for grids whose axes all have at most 64 points: any sizes, odd and unequal ones
+// among them, one CTA a unit of each chain.
+//
+// Waiting for the previous launch costs these grids as much as their work, so
+//   - two CTAs fit an SM (128 registers): those of phase k copy the operators and wait beside
+//     those of phase k - 1;
+//   - phi is summed in that time.  Phase k - 2 has completed when phase k starts to run (phase
+//     k - 1 lets it start only after its own wait), so the slots that phase finished are multiplied
+//     with the other chain's, stored long ago (second half of the contour).  The sums alternate
+//     between two accumulators with the parity of k, because those of phase k - 1 may still be on
+//     their way.
+// Per iteration on one B200 against what ran these grids before: 16^3 0.186 ms (persistent kernel
+// 0.331), 32^3 0.28 (0.46), 64^3 1.36 (1.46; P1 1.22 against 1.66), 200 steps of 45^3 P1 1.39 (three
+// passes a step 2.13).  A 64^3 phase takes 5.9 us: 4.3 in the CTA (2.4 of DMMA at the peak rate),
+// the rest from one launch's last store to the next one's first load.  The same phases as one
+// persistent launch with a release flag per unit pair took 9.1 us (4.5 of them until the last of a
+// CTA's 64 flags was seen), and so did holding back the q stores behind the release.
+// ---------------------------------------------------------------------------
+constexpr int kStepMaxN = 64;
+constexpr int kStepThreads = 256;
+constexpr int kStepResults = 16;  // results of a lane in one operation
+
+// phi work of one phase: acc += q qc of up to two slots (null pointers: none)
+struct PhiStep {
+    const double* q[2];
+    const double* qc[2];
+    double* acc[2];
+    int add[2];  // 0: the first term of this accumulator
+};
+
+struct ContourAnyArgs {
+    const double* in[2];   // k = 0: the initial slice; else the exchange buffer of the other layout
+    double* q[2];          // k >= 1: the finished slice
+    double* xout[2];       // k < U: this layout's exchange buffer, [x][y][zpad]
+    const double* w0[2];   // k >= 1: Boltzmann factor of the finished step
+    const double* w1[2];   // k < U: of the started step
+    const double* opz;     // packed blocks of A_z and of the layout's column axis
+    const double* opc;
+    int opz_count, opc_count;
+    int n[3];
+    int nchain, plane, finish, start;
+    int vec;               // 1: nz even and every array 16-byte aligned
+    PhiStep phi;
+};
+
+__host__ __device__ inline int step_zpad(int nz) { return (nz + 1) & ~1; }
+__host__ __device__ inline int step_ld(int nz) { return ((nz + 7) & ~7) + 4; }
+
+// Axis operations of a unit in block form MODE: kEo1 with run-time lengths (NC = 0) or on a cubic
+// grid of side NC; kEo2 / kCirc4 with NC = 64.
+template <int MODE, int NC>
+struct StepOp {
+    static constexpr int VPI = MODE == kEo1 ? 2 : 4;
+    static constexpr int NMAX = NC ? NC : kStepMaxN;
+    static constexpr int G = (NMAX + 8 * VPI - 1) / (8 * VPI);
+    static constexpr int ACC = MODE == kEo1 ? 2 : 4;
+    static_assert(G * 2 * VPI <= kStepResults, "results of a lane");
+    using Acc = double[ACC][G][1][2];
+
+    template <bool ROW>
+    __device__ __forceinline__ static void run(const double* T, int lf, const double* op, int n, int line0, Acc& acc) {
+        if constexpr (MODE != kEo1) {
+            warp_axis_mma<MODE, NC, 1, ROW>(T, op, line0, acc);
+        } else {
+            const int nn = NC ? NC : n, h = (nn + 1) / 2, hp = (h + 7) & ~7, ld = hp + 4, groups = hp / 8;
+            const int LF = NC ? NC + 4 : lf;
+            const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+            for (int r = 0; r < G; ++r)
+                acc[0][r][0][0] = acc[0][r][0][1] = acc[1][r][0][0] = acc[1][r][0][1] = 0.0;
+            const double* f = ROW ? T + (line0 + g) * LF : T + line0 + g;
+            const int KS = ROW ? 1 : LF;
+            const double* B = op + g * ld + t;
+#pragma unroll(NC ? 8 : 2)
+            for (int k0 = 0; k0 < hp; k0 += 4) {
+                const int j = k0 + t, jc = NC || j < h ? j : h - 1;  // padding columns of the operator are 0
+                const double x0 = f[jc * KS], x1 = f[(nn - 1 - jc) * KS];
+                const double u = x0 + x1, v = x0 - x1;
+#pragma unroll
+                for (int r = 0; r < G; ++r) {
+                    if (!NC && r >= groups) continue;
+                    const double e = B[8 * r * ld + k0], o = B[hp * ld + 8 * r * ld + k0];
+                    if (ROW) {
+                        dmma884(acc[0][r][0], u, e);
+                        dmma884(acc[1][r][0], v, o);
+                    } else {
+                        dmma884(acc[0][r][0], e, u);
+                        dmma884(acc[1][r][0], o, v);
+                    }
+                }
+            }
+        }
+    }
+    // results of group r, accumulator element e
+    __device__ __forceinline__ static void results(const Acc& acc, int r, int e, double (&y)[VPI]) {
+        if constexpr (MODE == kEo1) {
+            y[0] = acc[0][r][0][e] + acc[1][r][0][e];
+            y[1] = acc[0][r][0][e] - acc[1][r][0][e];
+        } else {
+            pair_results<MODE>(acc[0][r][0][e], acc[1][r][0][e], acc[2][r][0][e], acc[3][r][0][e], y);
+        }
+    }
+    // position k of pair index i; -1: none (padding, or the middle point a second time)
+    __device__ __forceinline__ static int position(int i, int k, int n) {
+        const int nn = NC ? NC : n;
+        if constexpr (MODE == kEo1) {
+            if (!NC && (2 * i > nn - 1 || (k == 1 && 2 * i == nn - 1))) return -1;
+            return k == 0 ? i : nn - 1 - i;
+        } else {
+            return k == 0 ? i : (k == 1 ? nn - 1 - i : (k == 2 ? nn / 2 - 1 - i : nn / 2 + i));
+        }
+    }
+};
+
+// acc += q qc over all points, by the whole grid
+__device__ __forceinline__ void phi_step(const PhiStep& p, long long M) {
+    if (!p.acc[0] && !p.acc[1]) return;
+    const bool one = p.acc[0] == p.acc[1];  // both slots in one block of the copolymer
+    const long long stride = (long long)gridDim.x * blockDim.x;
+#pragma unroll 4
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M; i += stride) {
+        const double a = p.acc[0] ? __ldcg(p.q[0] + i) * __ldcg(p.qc[0] + i) : 0.0;
+        const double b = p.acc[1] ? __ldcg(p.q[1] + i) * __ldcg(p.qc[1] + i) : 0.0;
+        if (one) {
+            __stcg(p.acc[0] + i, (p.add[0] ? __ldcg(p.acc[0] + i) : 0.0) + a + b);
+        } else {
+            if (p.acc[0]) __stcg(p.acc[0] + i, (p.add[0] ? __ldcg(p.acc[0] + i) : 0.0) + a);
+            if (p.acc[1]) __stcg(p.acc[1] + i, (p.add[1] ? __ldcg(p.acc[1] + i) : 0.0) + b);
+        }
+    }
+}
+
+template <int MODE, int NC>
+__global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const ContourAnyArgs a) {
+    using Op = StepOp<MODE, NC>;
+    constexpr int VPI = Op::VPI, G = Op::G;
+    const int nx = NC ? NC : a.n[0], ny = NC ? NC : a.n[1], nz = NC ? NC : a.n[2];
+    const int LF = NC ? NC + 4 : step_ld(nz), zpad = step_zpad(nz);
+    const bool plane = a.plane != 0;
+    const int R = plane ? ny : nx;  // rows of the tile; its columns are z
+    extern __shared__ __align__(16) double any[];
+    double* T = any;
+    double* opz = any + ((R + 7) & ~7) * LF;
+    double* opc = a.opc == a.opz ? opz : opz + a.opz_count;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g = lane >> 2, t = lane & 3, line0 = warp * 8;
+    for (int i = threadIdx.x; i < a.opz_count / 2; i += kStepThreads) cp_async16(opz + 2 * i, a.opz + 2 * i);
+    if (opc != opz)
+        for (int i = threadIdx.x; i < a.opc_count / 2; i += kStepThreads) cp_async16(opc + 2 * i, a.opc + 2 * i);
+    cp_async_commit();
+    phi_step(a.phi, (long long)nx * ny * nz);
+    cp_async_wait_all();
+    pdl_wait();
+    pdl_launch_dependents();
+    __syncthreads();  // the operators
+
+    const int units = nx > ny ? nx : ny;
+    const int c = (int)blockIdx.x >= units ? 1 : 0, p = (int)blockIdx.x - c * units;
+    if (!NC && p >= (plane ? nx : ny)) return;  // no unit in this layout
+    const long long psz = (long long)ny * nz, xpsz = (long long)ny * zpad;
+    const long long off = plane ? p * psz : (long long)p * nz, gs = plane ? nz : psz;
+    const long long xoff = plane ? p * xpsz : (long long)p * zpad, xgs = plane ? zpad : xpsz;
+    const bool warp_rows = line0 < R, warp_cols = line0 < nz;
+    const int col = line0 + 2 * t;  // this lane's columns: col, col + 1
+    const bool vec = NC || a.vec;
+    auto ld2 = [&](const double* s) {
+        if (vec) return __ldcg(reinterpret_cast<const double2*>(s));
+        return make_double2(__ldcg(s), col + 1 < nz ? __ldcg(s + 1) : 0.0);
+    };
+    // factors at this lane's column results, (group, point) order
+    double2 f[G * VPI];
+    auto factors = [&](const double* w) {
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+#pragma unroll
+            for (int k = 0; k < VPI; ++k) {
+                const int row = Op::position(8 * r + g, k, R);
+                f[r * VPI + k] = row >= 0 && col < nz ? ld2(w + row * gs + col) : make_double2(0.0, 0.0);
+            }
+    };
+    const double* in = c ? a.in[1] : a.in[0];
+    typename Op::Acc acc;
+    if (a.finish) {
+        // this warp's rows, A_z on them
+        if (warp_rows) {
+            const int r = line0 + g;
+            if (NC || r < R) {
+                const double* src = in + xoff + r * xgs;
+#pragma unroll(NC ? 8 : 4)
+                for (int ch = t; ch < zpad / 2; ch += 4) cp_async16(T + r * LF + 2 * ch, src + 2 * ch);
+                cp_async_commit();
+                cp_async_wait_all();
+            }
+            __syncwarp();
+            Op::template run<true>(T, LF, opz, nz, line0, acc);
+            __syncwarp();
+#pragma unroll
+            for (int r4 = 0; r4 < G; ++r4) {
+                double y0[VPI], y1[VPI];
+                Op::results(acc, r4, 0, y0);
+                Op::results(acc, r4, 1, y1);
+                double* row = T + (line0 + g) * LF;
+                const int i = 8 * r4 + 2 * t;
+#pragma unroll
+                for (int k = 0; k < VPI; ++k) {
+                    const int p0 = Op::position(i, k, nz), p1 = Op::position(i + 1, k, nz);
+                    if (NC) {
+                        *reinterpret_cast<double2*>(row + (p0 < p1 ? p0 : p1)) =
+                            p0 < p1 ? make_double2(y0[k], y1[k]) : make_double2(y1[k], y0[k]);
+                    } else {
+                        if (p0 >= 0) row[p0] = y0[k];
+                        if (p1 >= 0) row[p1] = y1[k];
+                    }
+                }
+            }
+        }
+        __syncthreads();  // every row is through A_z
+        if (!warp_cols) return;
+        const double* w0 = (c ? a.w0[1] : a.w0[0]) + off;
+        const double* w1 = a.start ? (c ? a.w1[1] : a.w1[0]) + off : w0;
+        factors(w0);  // in flight during the operation
+        Op::template run<false>(T, LF, opc, R, line0, acc);
+        __syncwarp();
+        double* q = (c ? a.q[1] : a.q[0]) + off;
+        double v[G * VPI][2];
+#pragma unroll
+        for (int r = 0; r < G; ++r) {
+            double y0[VPI], y1[VPI];
+            Op::results(acc, r, 0, y0);
+            Op::results(acc, r, 1, y1);
+#pragma unroll
+            for (int k = 0; k < VPI; ++k) {
+                const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
+                v[id][0] = y0[k] * f[id].x;
+                v[id][1] = y1[k] * f[id].y;
+                if (row < 0 || col >= nz) continue;
+                if (vec) {
+                    __stcg(reinterpret_cast<double2*>(q + row * gs + col), make_double2(v[id][0], v[id][1]));
+                } else {
+                    __stcg(q + row * gs + col, v[id][0]);
+                    if (col + 1 < nz) __stcg(q + row * gs + col + 1, v[id][1]);
+                }
+            }
+        }
+        if (w1 != w0) factors(w1);  // the step that starts is the first of the other block
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+#pragma unroll
+            for (int k = 0; k < VPI; ++k) {
+                const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
+                if (row >= 0)
+                    *reinterpret_cast<double2*>(T + row * LF + col) = make_double2(v[id][0] * f[id].x, v[id][1] * f[id].y);
+            }
+        __syncwarp();
+    } else {
+        // the first phase: D q(0), each warp its columns
+        if (!warp_cols) return;
+        factors((c ? a.w1[1] : a.w1[0]) + off);
+        const double* src = in + off;
+#pragma unroll
+        for (int r = 0; r < G; ++r)
+#pragma unroll
+            for (int k = 0; k < VPI; ++k) {
+                const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
+                if (row < 0) continue;
+                const double2 x = col < nz ? ld2(src + row * gs + col) : make_double2(0.0, 0.0);
+                *reinterpret_cast<double2*>(T + row * LF + col) = make_double2(x.x * f[id].x, x.y * f[id].y);
+            }
+        __syncwarp();
+    }
+    if (!a.start) return;
+    Op::template run<false>(T, LF, opc, R, line0, acc);
+    double* x = (c ? a.xout[1] : a.xout[0]) + xoff;
+#pragma unroll
+    for (int r = 0; r < G; ++r) {
+        double y0[VPI], y1[VPI];
+        Op::results(acc, r, 0, y0);
+        Op::results(acc, r, 1, y1);
+#pragma unroll
+        for (int k = 0; k < VPI; ++k) {
+            const int row = Op::position(8 * r + g, k, R);
+            if (row >= 0 && col < zpad)  // the padding column takes a dead value
+                __stcg(reinterpret_cast<double2*>(x + row * xgs + col), make_double2(y0[k], y1[k]));
+        }
     }
 }
 

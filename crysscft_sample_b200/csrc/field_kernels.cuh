@@ -264,6 +264,39 @@ __global__ void phi_fused_finish_kernel(const double* __restrict__ acc, const T*
     }
 }
 
+// phi from the sums of contour_any_kernel: acc[parity][block][point], contour order (null: no slot
+// went there), plus the slots `sp` that the sums leave out, with the trapezoid weights of
+// integrate_phi.
+struct PhiSlots {
+    const double* acc[2][2];
+    int count;
+    long long s[8];
+};
+__global__ void phi_step_finish_kernel(const double* __restrict__ q, const double* __restrict__ qc,
+                                       double* __restrict__ phiA, double* __restrict__ phiB, const IterState* st,
+                                       double fA, long long NsA, long long NsB, long long M, PhiSlots sp, PointOrder po) {
+    const long long U = NsA + NsB;
+    const double Q = st->Q;
+    const double cA = fA / (NsA * Q), cB = (1 - fA) / (NsB * Q);
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M; i += (long long)gridDim.x * blockDim.x) {
+        double s[2] = {0.0, 0.0};
+#pragma unroll
+        for (int b = 0; b < 2; ++b)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                if (sp.acc[h][b]) s[b] += sp.acc[h][b][i];
+        for (int j = 0; j < sp.count; ++j) {
+            const long long u = sp.s[j];
+            const double w = q[u * M + i] * qc[u * M + i];
+            if (u <= NsA) s[0] += (u == 0 || u == NsA ? 0.5 : 1.0) * w;
+            if (u >= NsA) s[1] += (u == NsA || u == U ? 0.5 : 1.0) * w;
+        }
+        const long long f = po.to_field(i);
+        phiA[f] = cA * s[0];
+        phiB[f] = cB * s[1];
+    }
+}
+
 __global__ void __launch_bounds__(kRedThreads)
 energy_kernel(const double* __restrict__ wA, const double* __restrict__ wB,
               const double* __restrict__ phiA, const double* __restrict__ phiB,

@@ -191,6 +191,7 @@ struct OpsSet {
         size_t off = 0;
     };
     Mma mma[3], dmma[3];
+    Mma one[3];  // axes within kStepMaxN in form kEo1 (contour_any_kernel), in d_mma; mode -1: none
     DevBuf<double> d_mma, d_dmma;
     static std::vector<const Mma*> before(const Mma* axes, int ax) {
         std::vector<const Mma*> e;
@@ -460,13 +461,11 @@ bool same(long double a, long double b) { return fabsl(a - b) <= 1e-17L * (1.0L 
 
 // Append one axis operator (n <= kMmaMaxN) in the block form of axis_mma.cuh its symmetry
 // allows.  perm: A is in 3m order (the pass reads and writes its points in that order).
-// earlier: the axes already packed into the same buffer.
+// earlier: the axes already packed into the same buffer.  one_level: kEo1 or nothing.
 void pack_operator_mma(const std::vector<long double>& A0, int n, bool perm, OpsSet::Mma& m, std::vector<double>& packed,
-                       const std::vector<const OpsSet::Mma*>& earlier) {
+                       const std::vector<const OpsSet::Mma*>& earlier, bool one_level = false) {
     m = OpsSet::Mma{};
     if (n > kMmaMaxN) return;
-    m.n = n;
-    m.perm = perm ? 1 : 0;
     auto at = [&](int j) { return !perm ? j : ((j & 1) ? n - 1 - (j >> 1) : (j >> 1)); };
     auto A = [&](int i, int j) { return A0[(size_t)at(i) * n + at(j)]; };
     bool centro = true;
@@ -474,7 +473,8 @@ void pack_operator_mma(const std::vector<long double>& A0, int n, bool perm, Ops
         for (int j = 0; centro && j < n; ++j) centro = same(A(i, j), A(n - 1 - i, n - 1 - j));
     const int half = n / 2;
     // two-level forms: only for the lengths with a specialised kernel (64, 96, 128)
-    bool eo2 = centro && n % 32 == 0 && n >= 64, circ = eo2;
+    if (one_level && !centro) return;  // m.mode stays -1
+    bool eo2 = !one_level && centro && n % 32 == 0 && n >= 64, circ = eo2;
     auto E = [&](int i, int j) { return (A(i, j) + A(i, n - 1 - j)) / 2; };
     for (int i = 0; i < half && (eo2 || circ); ++i)
         for (int j = 0; j < half && (eo2 || circ); ++j) {
@@ -483,6 +483,8 @@ void pack_operator_mma(const std::vector<long double>& A0, int n, bool perm, Ops
                    same(A(i, j), A(half - 1 - i, half - 1 - j)) &&
                    same(A(i, j + half), A(half - 1 - i, n - 1 - j));
         }
+    m.n = n;
+    m.perm = perm ? 1 : 0;
     m.mode = circ ? kCirc4 : (eo2 ? kEo2 : (centro ? kEo1 : kFull));
     const AxisBlocks b(m.mode, n);
     m.off = packed.size();
@@ -627,8 +629,6 @@ ContourStepFn contour_step_kernel_for(int mode, int n, bool one_op, int* threads
     CRYSSCFT_STEP(kEo2, 96, 1)
     CRYSSCFT_STEP(kCirc4, 128, 2)
     CRYSSCFT_STEP(kCirc4, 96, 1)
-    CRYSSCFT_STEP(kEo2, 64, 1)
-    CRYSSCFT_STEP(kCirc4, 64, 1)
 #undef CRYSSCFT_STEP
     *smem = 0;
     return nullptr;
@@ -790,6 +790,7 @@ struct scft_solver_s {
     M3Symmetry m3sym;                 // 3m mirror translations (decoded translational_part)
     std::vector<M3Term> m3terms;      // its Kronecker terms (one when the translations are 0)
     DevBuf<double> d_t3;              // input copy for in-place triplets of multi-term operators
+    DevBuf<double> d_x;               // exchange buffers of chains by contour_any_kernel
 
     ~scft_solver_s() {
         if (iomat) cudaFreeHost(iomat);
@@ -935,6 +936,119 @@ struct scft_solver_s {
         return SCFT_OK;
     }
 
+    // The launch of contour_any_kernel on this grid (fn null: it does not apply): single-term
+    // operators, every axis within kStepMaxN points, fields in the point order of the operators.
+    struct AnyPlan {
+        void (*fn)(const ContourAnyArgs) = nullptr;
+        const OpsSet::Mma* axes = nullptr;
+        size_t smem = 0;
+        size_t x_count = 0;  // doubles of one exchange buffer
+        bool fixed = false;  // a cubic side of its own kernel: 16-byte aligned arrays needed
+    };
+    AnyPlan any_plan(bool in_positions) const {
+        AnyPlan fp;
+        const OpsSet* o = ops;
+        if (!o || o->nterms != 1 || axis_form_override() != 0) return fp;
+        for (int ax = 0; ax < 3; ++ax)
+            if (o->one[ax].mode < 0 || (o->one[ax].perm && !in_positions)) return fp;
+        const int nx = (int)grid_phy[0], ny = (int)grid_phy[1], nz = (int)grid_phy[2];
+        const bool cubic = nx == ny && ny == nz;
+        const int m = o->mma[0].mode == o->mma[1].mode && o->mma[1].mode == o->mma[2].mode ? o->mma[0].mode : -1;
+        const bool two = cubic && nx == 64 && (m == kEo2 || m == kCirc4);
+        fp.axes = two ? o->mma : o->one;
+        fp.fixed = two || (cubic && (nx == 16 || nx == 32 || nx == 48));
+        fp.fn = two ? (m == kEo2 ? contour_any_kernel<kEo2, 64> : contour_any_kernel<kCirc4, 64>)
+                    : (!fp.fixed    ? contour_any_kernel<kEo1, 0>
+                       : nx == 16 ? contour_any_kernel<kEo1, 16>
+                       : nx == 32 ? contour_any_kernel<kEo1, 32>
+                                  : contour_any_kernel<kEo1, 48>);
+        size_t words = (size_t)((std::max(nx, ny) + 7) & ~7) * step_ld(nz);
+        const size_t cz = (size_t)AxisBlocks(fp.axes[2].mode, nz).count;
+        const size_t cy = (size_t)AxisBlocks(fp.axes[1].mode, ny).count, cx = (size_t)AxisBlocks(fp.axes[0].mode, nx).count;
+        fp.smem = (words + cz + std::max(cx, cy)) * sizeof(double);
+        fp.x_count = (size_t)nx * ny * step_zpad(nz);
+        return fp;
+    }
+
+    // U contour steps of nchain chains by contour_any_kernel, one launch per phase; segments < NsA
+    // take w[0], the rest w[1]; x: exchange buffers [layout][chain] of x_count doubles each.
+    // phi_acc (two chains over one contour): 4 fields for the sums of q q+; *sums: where they are and
+    // the slots they leave out.
+    int contour_any(const AnyPlan& fp, int nchain, const ChainSpan* ch, const double* const w[2], long long NsA, size_t U,
+                    double* x, double* phi_acc, PhiSlots* sums, cudaStream_t st) {
+        int grid = 1;
+        CKR(grant_pass((const void*)fp.fn, kStepThreads, fp.smem, &grid));
+        const int nx = (int)grid_phy[0], ny = (int)grid_phy[1], nz = (int)grid_phy[2];
+        const long long U_ = (long long)U, M_ = (long long)M;
+        auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+        bool vec = nz % 2 == 0 && aligned(w[0]) && aligned(w[1]);
+        for (int c = 0; c < nchain; ++c) vec = vec && aligned(ch[c].q);
+        auto factor = [&](const ChainSpan& c, long long step) {
+            const long long slot = c.slot0 + c.dir * step;
+            return w[(c.dir > 0 ? slot : slot - 1) < NsA ? 0 : 1];
+        };
+        std::vector<char> summed((size_t)U + 1, 0);
+        if (sums) *sums = PhiSlots{};
+        for (long long k = 0; k <= U_; ++k) {
+            ContourAnyArgs a{};
+            a.plane = (k & 1) == 0;
+            a.nchain = nchain;
+            a.finish = k >= 1;
+            a.start = k < U_;
+            a.n[0] = nx;
+            a.n[1] = ny;
+            a.n[2] = nz;
+            a.vec = vec ? 1 : 0;
+            const OpsSet::Mma& mz = fp.axes[2];
+            const OpsSet::Mma& mc = fp.axes[a.plane ? 1 : 0];
+            a.opz = ops->d_mma.p + mz.off;
+            a.opc = ops->d_mma.p + mc.off;
+            a.opz_count = AxisBlocks(mz.mode, mz.n).count;
+            a.opc_count = AxisBlocks(mc.mode, mc.n).count;
+            for (int c = 0; c < nchain; ++c) {
+                double* slice = ch[c].q + (ch[c].slot0 + ch[c].dir * k) * M_;
+                a.in[c] = k == 0 ? slice : x + (size_t)((a.plane ? 2 : 0) + c) * fp.x_count;
+                a.q[c] = slice;
+                a.xout[c] = x + (size_t)((a.plane ? 0 : 2) + c) * fp.x_count;
+                if (a.finish) a.w0[c] = factor(ch[c], k - 1);
+                if (a.start) a.w1[c] = factor(ch[c], k);
+            }
+            // the slots finished two phases ago, if the other chain has them too (see the kernel)
+            const long long kf = k - 2;
+            if (phi_acc && kf >= 1 && 2 * kf - U_ >= 2) {
+                for (int c = 0; c < 2; ++c) {
+                    const long long s = c == 0 ? kf : U_ - kf;
+                    if (s == NsA) continue;
+                    const int blk = s < NsA ? 0 : 1, h = (int)(k & 1);
+                    double* acc = phi_acc + (size_t)(2 * h + blk) * M;
+                    a.phi.q[c] = ch[0].q + s * M_;
+                    a.phi.qc[c] = ch[1].q + s * M_;
+                    a.phi.acc[c] = acc;
+                    a.phi.add[c] = sums->acc[h][blk] != nullptr;
+                    summed[(size_t)s] = 1;
+                }
+                for (int c = 0; c < 2; ++c)
+                    if (a.phi.acc[c]) sums->acc[(int)(k & 1)][a.phi.acc[c] == phi_acc + (size_t)(2 * (k & 1)) * M ? 0 : 1] = a.phi.acc[c];
+            }
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)(nchain * std::max(nx, ny)));
+            cfg.blockDim = dim3(kStepThreads);
+            cfg.dynamicSmemBytes = fp.smem;
+            cfg.stream = st;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            CK(cudaLaunchKernelEx(&cfg, fp.fn, a));
+            ++launches;
+        }
+        if (phi_acc)  // at most 8: 0, 1, U - 1, U, NsA and the middle one or two
+            for (long long s = 0; s <= U_; ++s)
+                if (!summed[(size_t)s]) sums->s[sums->count++] = s;
+        return SCFT_OK;
+    }
+
     // whether the FP32 tensor-core axis passes (axis_dmma.cuh, 3xTF32) run this grid by default,
     // on a cubic grid with a side the kernels cover (96 or 128), from measurements on one B200:
     // PMMM always; P1 for both chains of an iteration (128^3: 69.7 against 62.1 iterations/s) but
@@ -1066,6 +1180,8 @@ struct scft_solver_s {
             }
             CKR(upload_operator(A, (int)grid_phy[ax], *s, ax));
             pack_operator_mma(A, (int)grid_phy[ax], m3_plain, s->mma[ax], h_mma[0], OpsSet::before(s->mma, ax));
+            if (nt == 1 && grid_phy[ax] <= (size_t)kStepMaxN)
+                pack_operator_mma(A, (int)grid_phy[ax], m3_plain, s->one[ax], h_mma[0], OpsSet::before(s->one, ax), true);
             pack_operator(s->pos_order ? position_order(A, (int)grid_phy[ax]) : A, (int)grid_phy[ax], *s, ax);
             pack_operator_f32(A, (int)grid_phy[ax], *s, ax);
             if (nt == 1 && s->h16_axes == ax) pack_operator_h16(A, (int)grid_phy[ax], *s);
@@ -1297,6 +1413,7 @@ struct scft_diblock_s {
     ContourFn contour_fn = nullptr;
     bool alternating = false;             // contour_fn is the alternating-layout kernel
     bool alt_eo2 = false;                 // ... in its two-level even/odd form (operators d_packed2)
+    scft_solver_s::AnyPlan any_fp;        // FP64 contour by contour_any_kernel (fn null: not)
     int force_form = 0;                   // 0 auto, 1 alternating, 2 two-phase, 3 per-axis kernels
     int last_form = 0;                    // force_form the current launch plan was built with
     DevBuf<double> d_xch;                 // exchange buffers, 2 x space_size_phy per chain
@@ -1311,7 +1428,8 @@ struct scft_diblock_s {
     bool cluster_f32 = false;             // FP32 runs on the cluster kernel (contour_cluster_f32.cuh)
     DevBuf<float> f_xch;                  // FP32 exchange buffers
     DevBuf<unsigned> ctrl;                // [0] barrier arrivals, [1] error bits
-    long long spin_limit = 20000000LL;
+    static constexpr long long kSpinLimit = 20000000LL;
+    long long spin_limit = kSpinLimit;
 
     // graphs of the precision not in use (see scft_diblock_set_precision)
     cudaGraph_t saved_graph[2] = {nullptr, nullptr};
@@ -1508,6 +1626,20 @@ struct scft_diblock_s {
         return SCFT_OK;
     }
 
+    // Buffers of an iteration launched step by step (contour_any_kernel), before any capture.
+    int setup_any() {
+        any_fp = solver->any_plan(solver->ops && solver->ops->pos_order);
+        if (!any_fp.fn) return SCFT_OK;
+        if (d_xch.n < 4 * any_fp.x_count) CKR(d_xch.alloc(std::max(4 * M, 4 * any_fp.x_count)));
+        if (any_phi() && phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
+        return SCFT_OK;
+    }
+    // Whether contour_any_kernel sums phi itself: up to 2^16 points, where the sums fit into the
+    // wait for the previous launch (16^3 0.186 against 0.202 ms an iteration with the separate
+    // pass, 24^3 0.401 / 0.424, 40^3 1.24 / 1.30); on larger grids they reach into the launch they
+    // wait for (45^3 1.43 / 1.39, 64^3 1.67 / 1.36 ms).
+    bool any_phi() const { return fused_phi && M <= 65536; }
+
     int setup_persistent() {
         persistent = false;
         alternating = false;
@@ -1515,6 +1647,12 @@ struct scft_diblock_s {
         if (force_form == 3) return SCFT_OK;  // per-axis kernels only
         if (solver->ops && solver->ops->nterms > 1) return SCFT_OK;  // multi-term: per-axis kernels
         if (precision == SCFT_FP32) return setup_persistent_f32();
+        any_fp = {};
+        // (a caller's own poll limit asks for the kernels that wait)
+        if (force_form == 0 && spin_limit == kSpinLimit) {
+            CKR(setup_any());
+            if (any_fp.fn) return SCFT_OK;
+        }
         const OpsSet* o = solver->ops;
         if (!o) return SCFT_OK;
         for (int ax = 0; ax < 3; ++ax) {
@@ -1542,7 +1680,7 @@ struct scft_diblock_s {
                 alt_eo2 = false;
             }
         }
-        if (!d_xch.p) CKR(d_xch.alloc(4 * M));
+        if (d_xch.n < 4 * M) CKR(d_xch.alloc(4 * M));
         if (alternating && flags.n != alt_flag_count(nx)) CKR(flags.alloc(alt_flag_count(nx)));
         CK(cudaFuncSetAttribute(contour_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
@@ -1633,6 +1771,8 @@ struct scft_diblock_s {
         const int blocks = grid_blocks(MM, 256);
         size_t launches = 0;
         bool fused = false;  // phi was summed by this iteration's contour kernel
+        bool step_phi = false;  // ... of contour_any_kernel, whose sums are
+        PhiSlots step_sums{};
         PointOrder po{};
         if (sizeof(T) == 8 && solver->ops->pos_order) {
             po.on = 1;
@@ -1660,7 +1800,14 @@ struct scft_diblock_s {
             }
             bool stepped = false;
             if constexpr (sizeof(T) == 8) {
-                if (!persistent && solver->step_smem()) {
+                if (!persistent && any_fp.fn) {
+                    const ChainSpan ch[2] = {{q, 0, 1}, {qc, (long long)U, -1}};
+                    const double* w[2] = {wAds, wBds};
+                    CKR(solver->contour_any(any_fp, 2, ch, w, (long long)NsA, U, d_xch.p, any_phi() ? phi_acc.p : nullptr,
+                                            &step_sums, st));
+                    fused = step_phi = any_phi();
+                    stepped = true;
+                } else if (!persistent && solver->step_smem()) {
                     // each chain on a stream of its own: the launches of one chain fill the SMs that
                     // the other's leave (2 x 128 planes on 148 SMs are 1.73 rounds, not 2), and one
                     // chain's loads and stores run under the other's MMAs
@@ -1701,7 +1848,14 @@ struct scft_diblock_s {
         const int rblocks = (int)std::min<long long>(kRedMaxBlocks, (MM + kRedThreads - 1) / kRedThreads);
         q_reduce_kernel<T><<<rblocks, kRedThreads, 0, st>>>(qc, MM, partials.p, state.p);
         CK(cudaGetLastError());
-        if (fused)
+        if constexpr (sizeof(T) == 8) {
+            if (step_phi)
+                phi_step_finish_kernel<<<grid_blocks(MM, 256), 256, 0, st>>>(
+                    q, qc, phiA.p, phiB.p, state.p, fA, (long long)NsA, (long long)NsB, MM, step_sums, po);
+        }
+        if (step_phi) {
+            // done
+        } else if (fused)
             phi_fused_finish_kernel<T><<<grid_blocks(MM, 256), 256, 0, st>>>(
                 phi_acc.p, q, qc, phiA.p, phiB.p, state.p, fA, (long long)NsA, (long long)NsB,
                 (int)solver->grid_phy[0], po);
@@ -2037,12 +2191,17 @@ int scft_solver_propagate_device(scft_solver_t s, double* d_q, const double* d_i
     const size_t M = s->M;
     size_t slot = direction == 1 ? 0 : Ns;
     CK(cudaMemcpyAsync(d_q + slot * M, d_init, M * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    // one launch per step where the step kernel covers the grid; it moves 16-byte words, so the
-    // caller's arrays must be aligned to them (the three passes take any)
+    // one launch per step where a step kernel covers the grid; those for fixed sides move 16-byte
+    // words, so the caller's arrays must be aligned to them (the three passes take any)
     const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    const ChainSpan ch{d_q, (long long)slot, direction};
+    const double* w[2] = {d_wds, d_wds};
+    const auto any = s->any_plan(false);
+    if (Ns > 0 && any.fn && (!any.fixed || (aligned(d_q) && aligned(d_wds)))) {
+        if (s->d_x.n < 4 * any.x_count) CKR(s->d_x.alloc(4 * any.x_count));
+        return s->contour_any(any, 1, &ch, w, 0, Ns, s->d_x.p, nullptr, nullptr, st);
+    }
     if (Ns > 0 && !s->ops->mma[0].perm && aligned(d_q) && aligned(d_wds) && s->step_smem()) {
-        const ChainSpan ch{d_q, (long long)slot, direction};
-        const double* w[2] = {d_wds, d_wds};
         double* x[4] = {s->d_t1.p, nullptr, s->d_t2.p, nullptr};
         return s->contour_steps(1, &ch, w, 0, Ns, x, st);
     }
@@ -2909,7 +3068,8 @@ struct scft_batch_s {
 
     int build_graph() {
         drop_graph();
-        const int ff = form == 4 ? 0 : form;  // the instances' own plan under form 4: automatic
+        // form 4: the alternating kernel's plan where it applies (the batch kernel runs its schedule)
+        const int ff = form == 4 ? 1 : form;
         for (auto d : runs) {
             d->force_form = ff;
             if (d->captured_gen == d->solver->ops_gen && d->last_form != ff) d->captured_gen = ~0ULL;

@@ -209,21 +209,23 @@ int scft_diblock_get_precision(scft_diblock_t d, int* out);
  * The history is cleared by this call and by scft_diblock_set_fields. */
 int scft_diblock_set_mixing(scft_diblock_t d, int history, double beta);
 
-/* Poll limit of every bounded wait inside the contour kernels (release flags, grid
+/* Poll limit of every bounded wait inside the persistent contour kernels (release flags, grid
  * barriers, tile loads; default 20,000,000, about a second).  A wait that runs out makes
  * the kernel record an error, let its own copies land and return, and the iteration call
- * returns SCFT_ERR_TIMEOUT; the context stays usable.  No counterpart in the reference
+ * returns SCFT_ERR_TIMEOUT; the context stays usable.  FP64 iterations on grids of up to 64
+ * points a side run one launch per contour step, which waits on nothing; with a limit other
+ * than the default they run the persistent kernel where it covers the grid.  No counterpart in the reference
  * (it has no device code); a small limit is how the timeout path is tested. */
 int scft_diblock_set_wait_limit(scft_diblock_t d, long long spins);
 
-/* Where the FP64 iterations integrate phi_A and phi_B over the contour (integrate_phi,
+/* Where the iterations integrate phi_A and phi_B over the contour (integrate_phi,
  * src/crysSCFT_sample.cpp:348-360, trapezoid weights): fused = 1 (default) lets the
- * whole-contour kernel on cubic grids add q(s) q+(s) tile by tile as the second chain
- * reaches each slot, so a short kernel finishes phi instead of a pass over the stored
- * contour; fused = 0 always uses that separate pass.  The two agree to rounding (the sums
- * run in a different order).  The fused form applies to the alternating whole-contour
- * kernel with an even number of contour steps; other plans use the separate pass either
- * way.  No counterpart in the reference (a form switch of this library). */
+ * contour kernels add q(s) q+(s) as the second chain reaches each slot, so a short kernel
+ * finishes phi instead of a pass over the stored contour; fused = 0 always uses that
+ * separate pass.  The two agree to rounding (the sums run in a different order).  The
+ * fused form applies to FP64 grids of up to 65536 physical points and to the alternating
+ * whole-contour kernels with an even number of contour steps; other plans use the
+ * separate pass either way.  No counterpart in the reference (a form switch of this library). */
 int scft_diblock_set_phi_form(scft_diblock_t d, int fused);
 
 /* rms residual sqrt(<r, r> / 2M) of each iteration of the last scft_diblock_iterate
