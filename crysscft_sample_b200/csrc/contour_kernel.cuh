@@ -475,7 +475,9 @@ __device__ __forceinline__ void row_op_ct(const double* __restrict__ F, double* 
 // accumulators, so the stores overlap the other warps' tiles.
 // kFinish (two-level kernel): the result y finishes a contour step: q = y W0 goes to the
 // panel staging tile qs (stored from there by TMA) and, if start, q W1 to the slab G.
-enum ColEpilogue { kToSmem = 0, kToGlobal = 1, kFinish = 2 };
+// kFinishDirect (FP32 step kernel): as kFinish, with W0 and W1 in slabs like G and q stored to
+// global memory (qs, row stride gs).
+enum ColEpilogue { kToSmem = 0, kToGlobal = 1, kFinish = 2, kFinishDirect = 3 };
 
 struct ColOut {
     double* G;

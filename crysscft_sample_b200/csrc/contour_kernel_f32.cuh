@@ -180,6 +180,15 @@ __device__ __forceinline__ void col_store_f32(const ColOutF& o, int i, int c, fl
         *reinterpret_cast<float2*>(o.G + i * LF + c) = make_float2(v0, v1);
     } else if constexpr (EPI == kToGlobal) {
         *reinterpret_cast<float2*>(o.G + i * o.gs + c) = make_float2(v0, v1);
+    } else if constexpr (EPI == kFinishDirect) {
+        const float2 w0 = *reinterpret_cast<const float2*>(o.w0 + i * LF + c);
+        v0 = v0 * w0.x;
+        v1 = v1 * w0.y;
+        __stcg(reinterpret_cast<float2*>(o.qs + i * o.gs + c), make_float2(v0, v1));
+        if (o.start) {
+            const float2 w1 = *reinterpret_cast<const float2*>(o.w1 + i * LF + c);
+            *reinterpret_cast<float2*>(o.G + i * LF + c) = make_float2(v0 * w1.x, v1 * w1.y);
+        }
     } else {  // kFinish, as col_store
         const int pi = panel_index<PR>(i, c);
         const float2 w0 = *reinterpret_cast<const float2*>(o.w0 + pi);

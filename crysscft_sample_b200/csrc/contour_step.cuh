@@ -298,9 +298,10 @@ constexpr int kStepThreads = 256;
 constexpr int kStepResults = 16;  // results of a lane in one operation
 
 // phi work of one phase: acc += q qc of up to two slots (null pointers: none)
+template <typename T>
 struct PhiStep {
-    const double* q[2];
-    const double* qc[2];
+    const T* q[2];
+    const T* qc[2];
     double* acc[2];
     int add[2];  // 0: the first term of this accumulator
 };
@@ -317,7 +318,7 @@ struct ContourAnyArgs {
     int n[3];
     int nchain, plane, finish, start;
     int vec;               // 1: nz even and every array 16-byte aligned
-    PhiStep phi;
+    PhiStep<double> phi;
 };
 
 __host__ __device__ inline int step_zpad(int nz) { return (nz + 1) & ~1; }
@@ -390,14 +391,15 @@ struct StepOp {
 };
 
 // acc += q qc over all points, by the whole grid
-__device__ __forceinline__ void phi_step(const PhiStep& p, long long M) {
+template <typename T>
+__device__ __forceinline__ void phi_step(const PhiStep<T>& p, long long M) {
     if (!p.acc[0] && !p.acc[1]) return;
     const bool one = p.acc[0] == p.acc[1];  // both slots in one block of the copolymer
     const long long stride = (long long)gridDim.x * blockDim.x;
 #pragma unroll 4
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M; i += stride) {
-        const double a = p.acc[0] ? __ldcg(p.q[0] + i) * __ldcg(p.qc[0] + i) : 0.0;
-        const double b = p.acc[1] ? __ldcg(p.q[1] + i) * __ldcg(p.qc[1] + i) : 0.0;
+        const double a = p.acc[0] ? (double)__ldcg(p.q[0] + i) * (double)__ldcg(p.qc[0] + i) : 0.0;
+        const double b = p.acc[1] ? (double)__ldcg(p.q[1] + i) * (double)__ldcg(p.qc[1] + i) : 0.0;
         if (one) {
             __stcg(p.acc[0] + i, (p.add[0] ? __ldcg(p.acc[0] + i) : 0.0) + a + b);
         } else {

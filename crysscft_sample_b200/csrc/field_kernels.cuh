@@ -272,7 +272,8 @@ struct PhiSlots {
     int count;
     long long s[8];
 };
-__global__ void phi_step_finish_kernel(const double* __restrict__ q, const double* __restrict__ qc,
+template <typename T>
+__global__ void phi_step_finish_kernel(const T* __restrict__ q, const T* __restrict__ qc,
                                        double* __restrict__ phiA, double* __restrict__ phiB, const IterState* st,
                                        double fA, long long NsA, long long NsB, long long M, PhiSlots sp, PointOrder po) {
     const long long U = NsA + NsB;
@@ -287,7 +288,7 @@ __global__ void phi_step_finish_kernel(const double* __restrict__ q, const doubl
                 if (sp.acc[h][b]) s[b] += sp.acc[h][b][i];
         for (int j = 0; j < sp.count; ++j) {
             const long long u = sp.s[j];
-            const double w = q[u * M + i] * qc[u * M + i];
+            const double w = (double)q[u * M + i] * (double)qc[u * M + i];
             if (u <= NsA) s[0] += (u == 0 || u == NsA ? 0.5 : 1.0) * w;
             if (u >= NsA) s[1] += (u == NsA || u == U ? 0.5 : 1.0) * w;
         }

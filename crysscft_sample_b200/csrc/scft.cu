@@ -27,6 +27,7 @@
 #include "contour_batch.cuh"
 #include "contour_cluster_f32.cuh"
 #include "contour_step.cuh"
+#include "contour_step_f32.cuh"
 #include "contour_kernel_f32.cuh"
 #include "field_kernels.cuh"
 #include "operators.h"
@@ -688,6 +689,28 @@ ContourFnF contour_alt_kernel_f32_for(int n, int eo, size_t* smem) {
     return nullptr;
 }
 
+using ContourStepFnF = void (*)(const ContourStepArgsF);
+
+// The one-launch-per-phase form of contour_alt_kernel_f32; nullptr when there is none.
+ContourStepFnF contour_step_kernel_f32_for(int n, int eo, size_t* smem) {
+#define CRYSSCFT_STEPF(N, E)                   \
+    {                                          \
+        *smem = StepShapeF<N, E>::SMEM;        \
+        return contour_step_kernel_f32<N, E>;  \
+    }
+    if (eo) {
+        if (n == 32) CRYSSCFT_STEPF(32, true)
+        if (n == 64) CRYSSCFT_STEPF(64, true)
+    } else {
+        if (n == 16) CRYSSCFT_STEPF(16, false)
+        if (n == 32) CRYSSCFT_STEPF(32, false)
+        if (n == 48) CRYSSCFT_STEPF(48, false)
+        if (n == 64) CRYSSCFT_STEPF(64, false)
+    }
+#undef CRYSSCFT_STEPF
+    return nullptr;
+}
+
 ContourFn contour_alt_kernel_for(int n, int eo, size_t* smem, bool eo2 = false) {
     if (eo2 && eo && n == 64) {
         *smem = AltShape<64, true, true>::SMEM;
@@ -752,6 +775,45 @@ ContourFn contour_kernel_for(int nx, int ny, int nz, const int eo[3]) {
 }
 
 }  // namespace
+
+// Which slots the launch of phase k sums for phi (contour_any_kernel, contour_step_kernel_f32): those
+// that phase k - 2 finished, if the other chain has them too; slot NsA and the ones that no phase
+// takes go to `sums` for the finishing kernel (at most 8: 0, 1, U - 1, U, NsA and the middle one or
+// two).
+template <typename T>
+struct PhiSchedule {
+    const T* q;
+    const T* qc;
+    double* acc;  // 4 fields [parity of k][block]; null: phi is not summed
+    long long U, NsA, M;
+    PhiSlots sums{};
+    std::vector<char> summed;
+    PhiSchedule(const T* q_, const T* qc_, double* acc_, long long U_, long long NsA_, long long M_)
+        : q(q_), qc(qc_), acc(acc_), U(U_), NsA(NsA_), M(M_), summed((size_t)U_ + 1, 0) {}
+    PhiStep<T> of(long long k) {
+        PhiStep<T> p{};
+        const long long kf = k - 2;
+        if (!acc || kf < 1 || 2 * kf - U < 2) return p;
+        const int h = (int)(k & 1);
+        for (int c = 0; c < 2; ++c) {
+            const long long s = c == 0 ? kf : U - kf;
+            if (s == NsA) continue;
+            p.q[c] = q + s * M;
+            p.qc[c] = qc + s * M;
+            p.acc[c] = acc + (size_t)(2 * h + (s < NsA ? 0 : 1)) * M;
+            p.add[c] = sums.acc[h][s < NsA ? 0 : 1] != nullptr;
+            summed[(size_t)s] = 1;
+        }
+        for (int b = 0; b < 2; ++b)
+            for (int c = 0; c < 2; ++c)
+                if (p.acc[c] == acc + (size_t)(2 * h + b) * M) sums.acc[h][b] = p.acc[c];
+        return p;
+    }
+    void finish() {
+        for (long long s = 0; acc && s <= U; ++s)
+            if (!summed[(size_t)s]) sums.s[sums.count++] = s;
+    }
+};
 
 // One chain of contour steps over a store of slices: input slot slot0 + dir t of step t.
 struct ChainSpan {
@@ -972,10 +1034,9 @@ struct scft_solver_s {
 
     // U contour steps of nchain chains by contour_any_kernel, one launch per phase; segments < NsA
     // take w[0], the rest w[1]; x: exchange buffers [layout][chain] of x_count doubles each.
-    // phi_acc (two chains over one contour): 4 fields for the sums of q q+; *sums: where they are and
-    // the slots they leave out.
+    // phi (two chains over one contour, or null): the sums of q q+ on the way.
     int contour_any(const AnyPlan& fp, int nchain, const ChainSpan* ch, const double* const w[2], long long NsA, size_t U,
-                    double* x, double* phi_acc, PhiSlots* sums, cudaStream_t st) {
+                    double* x, PhiSchedule<double>* phi, cudaStream_t st) {
         int grid = 1;
         CKR(grant_pass((const void*)fp.fn, kStepThreads, fp.smem, &grid));
         const int nx = (int)grid_phy[0], ny = (int)grid_phy[1], nz = (int)grid_phy[2];
@@ -987,8 +1048,6 @@ struct scft_solver_s {
             const long long slot = c.slot0 + c.dir * step;
             return w[(c.dir > 0 ? slot : slot - 1) < NsA ? 0 : 1];
         };
-        std::vector<char> summed((size_t)U + 1, 0);
-        if (sums) *sums = PhiSlots{};
         for (long long k = 0; k <= U_; ++k) {
             ContourAnyArgs a{};
             a.plane = (k & 1) == 0;
@@ -1013,23 +1072,7 @@ struct scft_solver_s {
                 if (a.finish) a.w0[c] = factor(ch[c], k - 1);
                 if (a.start) a.w1[c] = factor(ch[c], k);
             }
-            // the slots finished two phases ago, if the other chain has them too (see the kernel)
-            const long long kf = k - 2;
-            if (phi_acc && kf >= 1 && 2 * kf - U_ >= 2) {
-                for (int c = 0; c < 2; ++c) {
-                    const long long s = c == 0 ? kf : U_ - kf;
-                    if (s == NsA) continue;
-                    const int blk = s < NsA ? 0 : 1, h = (int)(k & 1);
-                    double* acc = phi_acc + (size_t)(2 * h + blk) * M;
-                    a.phi.q[c] = ch[0].q + s * M_;
-                    a.phi.qc[c] = ch[1].q + s * M_;
-                    a.phi.acc[c] = acc;
-                    a.phi.add[c] = sums->acc[h][blk] != nullptr;
-                    summed[(size_t)s] = 1;
-                }
-                for (int c = 0; c < 2; ++c)
-                    if (a.phi.acc[c]) sums->acc[(int)(k & 1)][a.phi.acc[c] == phi_acc + (size_t)(2 * (k & 1)) * M ? 0 : 1] = a.phi.acc[c];
-            }
+            if (phi) a.phi = phi->of(k);
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = dim3((unsigned)(nchain * std::max(nx, ny)));
             cfg.blockDim = dim3(kStepThreads);
@@ -1043,9 +1086,7 @@ struct scft_solver_s {
             CK(cudaLaunchKernelEx(&cfg, fp.fn, a));
             ++launches;
         }
-        if (phi_acc)  // at most 8: 0, 1, U - 1, U, NsA and the middle one or two
-            for (long long s = 0; s <= U_; ++s)
-                if (!summed[(size_t)s]) sums->s[sums->count++] = s;
+        if (phi) phi->finish();
         return SCFT_OK;
     }
 
@@ -1413,6 +1454,8 @@ struct scft_diblock_s {
     ContourFn contour_fn = nullptr;
     bool alternating = false;             // contour_fn is the alternating-layout kernel
     bool alt_eo2 = false;                 // ... in its two-level even/odd form (operators d_packed2)
+    ContourStepFnF step_fn_f32 = nullptr; // FP32 contour one launch per phase (null: not)
+    size_t step_smem_f32 = 0;
     scft_solver_s::AnyPlan any_fp;        // FP64 contour by contour_any_kernel (fn null: not)
     int force_form = 0;                   // 0 auto, 1 alternating, 2 two-phase, 3 per-axis kernels
     int last_form = 0;                    // force_form the current launch plan was built with
@@ -1537,15 +1580,70 @@ struct scft_diblock_s {
         return SCFT_OK;
     }
 
+    // FP32 steps, one launch per phase (contour_step_f32.cuh)
+    int contour_steps_f32(cudaStream_t st, float* wAds, float* wBds, float* q, float* qc, PhiSchedule<float>& phi) {
+        const int n = (int)solver->grid_phy[0];
+        int grid = 1;
+        CKR(solver->grant_pass((const void*)step_fn_f32, kContourThreads, step_smem_f32, &grid));
+        float* store[2] = {q, qc};
+        const long long slot0[2] = {0, (long long)U}, dir[2] = {1, -1};
+        const float* w[2] = {wAds, wBds};
+        auto factor = [&](int c, long long step) {
+            const long long slot = slot0[c] + dir[c] * step;
+            return w[(dir[c] > 0 ? slot : slot - 1) < (long long)NsA ? 0 : 1];
+        };
+        for (long long k = 0; k <= (long long)U; ++k) {
+            ContourStepArgsF a{};
+            a.plane = (k & 1) == 0;
+            a.finish = k >= 1;
+            a.start = k < (long long)U;
+            a.ops = solver->ops->f_packed.p;
+            for (int c = 0; c < 2; ++c) {
+                float* slice = store[c] + (slot0[c] + dir[c] * k) * (long long)M;
+                float* xp = f_xch.p + (size_t)(2 * c) * M;  // XP, then XS
+                a.in[c] = k == 0 ? slice : (a.plane ? xp + M : xp);
+                a.q[c] = slice;
+                a.xout[c] = a.plane ? xp : xp + M;
+                if (a.finish) a.w0[c] = factor(c, k - 1);
+                if (a.start) a.w1[c] = factor(c, k);
+            }
+            a.phi = phi.of(k);
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3((unsigned)(2 * n));
+            cfg.blockDim = dim3(kContourThreads);
+            cfg.dynamicSmemBytes = step_smem_f32;
+            cfg.stream = st;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            attr[0].val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = attr;
+            cfg.numAttrs = 1;
+            CK(cudaLaunchKernelEx(&cfg, step_fn_f32, a));
+            ++solver->launches;
+        }
+        phi.finish();
+        return SCFT_OK;
+    }
+
     int setup_persistent_f32() {
         persistent = false;
         f32_phi_fused = false;
+        step_fn_f32 = nullptr;
         CKR(setup_cluster_f32());
         if (cluster_f32) return SCFT_OK;
         const OpsSet* o = solver->ops;
         if (!o) return SCFT_OK;
         const int nx = (int)solver->grid_phy[0], ny = (int)solver->grid_phy[1], nz = (int)solver->grid_phy[2];
         if (nx != ny || ny != nz || o->eo_f32[0] != o->eo_f32[1] || o->eo_f32[1] != o->eo_f32[2]) return SCFT_OK;
+        // (a caller's own poll limit asks for the kernels that wait)
+        if (force_form == 0 && spin_limit == kSpinLimit && axis_form_override() == 0) {
+            step_fn_f32 = contour_step_kernel_f32_for(nx, o->eo_f32[0], &step_smem_f32);
+            if (step_fn_f32) {
+                if (!f_xch.p) CKR(f_xch.alloc(4 * M));
+                if (any_phi() && phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
+                return SCFT_OK;
+            }
+        }
         size_t smem = 0;
         ContourFnF f = contour_alt_kernel_f32_for(nx, o->eo_f32[0], &smem);
         if (!f) return SCFT_OK;
@@ -1799,12 +1897,22 @@ struct scft_diblock_s {
                 ++solver->launches;
             }
             bool stepped = false;
+            if constexpr (sizeof(T) == 4) {
+                if (!persistent && step_fn_f32) {
+                    PhiSchedule<float> ps(q, qc, any_phi() ? phi_acc.p : nullptr, (long long)U, (long long)NsA, MM);
+                    CKR(contour_steps_f32(st, wAds, wBds, q, qc, ps));
+                    step_sums = ps.sums;
+                    fused = step_phi = any_phi();
+                    stepped = true;
+                }
+            }
             if constexpr (sizeof(T) == 8) {
                 if (!persistent && any_fp.fn) {
                     const ChainSpan ch[2] = {{q, 0, 1}, {qc, (long long)U, -1}};
                     const double* w[2] = {wAds, wBds};
-                    CKR(solver->contour_any(any_fp, 2, ch, w, (long long)NsA, U, d_xch.p, any_phi() ? phi_acc.p : nullptr,
-                                            &step_sums, st));
+                    PhiSchedule<double> ps(q, qc, any_phi() ? phi_acc.p : nullptr, (long long)U, (long long)NsA, MM);
+                    CKR(solver->contour_any(any_fp, 2, ch, w, (long long)NsA, U, d_xch.p, &ps, st));
+                    step_sums = ps.sums;
                     fused = step_phi = any_phi();
                     stepped = true;
                 } else if (!persistent && solver->step_smem()) {
@@ -1848,14 +1956,10 @@ struct scft_diblock_s {
         const int rblocks = (int)std::min<long long>(kRedMaxBlocks, (MM + kRedThreads - 1) / kRedThreads);
         q_reduce_kernel<T><<<rblocks, kRedThreads, 0, st>>>(qc, MM, partials.p, state.p);
         CK(cudaGetLastError());
-        if constexpr (sizeof(T) == 8) {
-            if (step_phi)
-                phi_step_finish_kernel<<<grid_blocks(MM, 256), 256, 0, st>>>(
-                    q, qc, phiA.p, phiB.p, state.p, fA, (long long)NsA, (long long)NsB, MM, step_sums, po);
-        }
-        if (step_phi) {
-            // done
-        } else if (fused)
+        if (step_phi)
+            phi_step_finish_kernel<T><<<grid_blocks(MM, 256), 256, 0, st>>>(
+                q, qc, phiA.p, phiB.p, state.p, fA, (long long)NsA, (long long)NsB, MM, step_sums, po);
+        else if (fused)
             phi_fused_finish_kernel<T><<<grid_blocks(MM, 256), 256, 0, st>>>(
                 phi_acc.p, q, qc, phiA.p, phiB.p, state.p, fA, (long long)NsA, (long long)NsB,
                 (int)solver->grid_phy[0], po);
@@ -2199,7 +2303,7 @@ int scft_solver_propagate_device(scft_solver_t s, double* d_q, const double* d_i
     const auto any = s->any_plan(false);
     if (Ns > 0 && any.fn && (!any.fixed || (aligned(d_q) && aligned(d_wds)))) {
         if (s->d_x.n < 4 * any.x_count) CKR(s->d_x.alloc(4 * any.x_count));
-        return s->contour_any(any, 1, &ch, w, 0, Ns, s->d_x.p, nullptr, nullptr, st);
+        return s->contour_any(any, 1, &ch, w, 0, Ns, s->d_x.p, nullptr, st);
     }
     if (Ns > 0 && !s->ops->mma[0].perm && aligned(d_q) && aligned(d_wds) && s->step_smem()) {
         double* x[4] = {s->d_t1.p, nullptr, s->d_t2.p, nullptr};
