@@ -28,6 +28,7 @@
 #include "contour_cluster_f32.cuh"
 #include "contour_step.cuh"
 #include "contour_step_f32.cuh"
+#include "contour_simt_f32.cuh"
 #include "contour_kernel_f32.cuh"
 #include "field_kernels.cuh"
 #include "operators.h"
@@ -1167,6 +1168,19 @@ struct scft_solver_s {
         return SCFT_OK;
     }
 
+    // whether an FP32 triplet on this grid is three SIMT passes (no FFT on some axis, no 3xTF32 passes)
+    // of axes that contour_simt_kernel_f32 holds
+    bool simt_steps_f32() const {
+        if (!ops || ops->nterms != 1 || axis_form_override() != 0) return false;
+        bool fft = true;
+        for (int ax = 0; ax < 3; ++ax) {
+            size_t smem = 0;
+            if (grid_phy[ax] > (size_t)kSimtMaxN) return false;
+            fft = fft && fft_kernel<float>(ax, &smem) != nullptr;
+        }
+        return !fft;
+    }
+
     // one SIMT pass (axis_kernels.cuh) along axis ax of term o
     template <typename T>
     int simt_pass(int ax, OpsSet* o, int nchain, const T* const in[2], T* const out[2], const T* const pre[2],
@@ -1456,6 +1470,7 @@ struct scft_diblock_s {
     bool alt_eo2 = false;                 // ... in its two-level even/odd form (operators d_packed2)
     ContourStepFnF step_fn_f32 = nullptr; // FP32 contour one launch per phase (null: not)
     size_t step_smem_f32 = 0;
+    bool simt_f32 = false;                // FP32 contour by contour_simt_kernel_f32
     scft_solver_s::AnyPlan any_fp;        // FP64 contour by contour_any_kernel (fn null: not)
     int force_form = 0;                   // 0 auto, 1 alternating, 2 two-phase, 3 per-axis kernels
     int last_form = 0;                    // force_form the current launch plan was built with
@@ -1625,15 +1640,69 @@ struct scft_diblock_s {
         return SCFT_OK;
     }
 
+    // FP32 steps of grids off the tensor-core sizes, two launches each (contour_simt_f32.cuh)
+    int contour_simt_f32(cudaStream_t st, float* wAds, float* wBds, float* q, float* qc, float* const x[2],
+                         PhiSchedule<float>& phi) {
+        const int nx = (int)solver->grid_phy[0], ny = (int)solver->grid_phy[1], nz = (int)solver->grid_phy[2];
+        const size_t smem = simt_smem(nx, ny, nz);
+        int grid = 1;
+        CKR(solver->grant_pass((const void*)contour_simt_kernel_f32, kSimtThreads, smem, &grid));
+        const OpsSet* o = solver->ops;
+        for (long long t = 0; t < (long long)U; ++t)
+            for (int half = 0; half < 2; ++half) {
+                ContourSimtArgsF a{};
+                a.plane = half == 0;
+                a.n[0] = nx;
+                a.n[1] = ny;
+                a.n[2] = nz;
+                a.opT[0] = o->f_opT[half == 0 ? 2 : 0].p;
+                a.opT[1] = o->f_opT[1].p;
+                const long long s0 = t, s1 = (long long)U - t;  // input slots of the chains
+                float* slice[2] = {q + (half == 0 ? s0 : s0 + 1) * (long long)M, qc + (half == 0 ? s1 : s1 - 1) * (long long)M};
+                for (int c = 0; c < 2; ++c) {
+                    a.in[c] = half == 0 ? slice[c] : x[c];
+                    a.out[c] = half == 0 ? x[c] : slice[c];
+                    a.w[c] = (c == 0 ? s0 : s1 - 1) < (long long)NsA ? wAds : wBds;
+                }
+                // the slab launch of step t - 2, which finished slot t - 1, is two launches back
+                if (half == 0) a.phi = phi.of(t + 1);
+                cudaLaunchConfig_t cfg{};
+                cfg.gridDim = dim3((unsigned)(2 * std::max(nx, ny)));
+                cfg.blockDim = dim3(kSimtThreads);
+                cfg.dynamicSmemBytes = smem;
+                cfg.stream = st;
+                cudaLaunchAttribute attr[1];
+                attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+                attr[0].val.programmaticStreamSerializationAllowed = 1;
+                cfg.attrs = attr;
+                cfg.numAttrs = 1;
+                CK(cudaLaunchKernelEx(&cfg, contour_simt_kernel_f32, a));
+                ++solver->launches;
+            }
+        phi.finish();
+        return SCFT_OK;
+    }
+
     int setup_persistent_f32() {
         persistent = false;
         f32_phi_fused = false;
         step_fn_f32 = nullptr;
+        simt_f32 = false;
         CKR(setup_cluster_f32());
         if (cluster_f32) return SCFT_OK;
         const OpsSet* o = solver->ops;
         if (!o) return SCFT_OK;
         const int nx = (int)solver->grid_phy[0], ny = (int)solver->grid_phy[1], nz = (int)solver->grid_phy[2];
+        {
+            size_t smem = 0;
+            const bool tiled = nx == ny && ny == nz && o->eo_f32[0] == o->eo_f32[1] && o->eo_f32[1] == o->eo_f32[2] &&
+                               contour_alt_kernel_f32_for(nx, o->eo_f32[0], &smem) != nullptr;
+            if (!tiled && solver->simt_steps_f32()) {
+                simt_f32 = true;
+                if (any_phi() && phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
+                return SCFT_OK;
+            }
+        }
         if (nx != ny || ny != nz || o->eo_f32[0] != o->eo_f32[1] || o->eo_f32[1] != o->eo_f32[2]) return SCFT_OK;
         // (a caller's own poll limit asks for the kernels that wait)
         if (force_form == 0 && spin_limit == kSpinLimit && axis_form_override() == 0) {
@@ -1898,9 +1967,10 @@ struct scft_diblock_s {
             }
             bool stepped = false;
             if constexpr (sizeof(T) == 4) {
-                if (!persistent && step_fn_f32) {
+                if (!persistent && (step_fn_f32 || simt_f32)) {
                     PhiSchedule<float> ps(q, qc, any_phi() ? phi_acc.p : nullptr, (long long)U, (long long)NsA, MM);
-                    CKR(contour_steps_f32(st, wAds, wBds, q, qc, ps));
+                    if (step_fn_f32) CKR(contour_steps_f32(st, wAds, wBds, q, qc, ps));
+                    else CKR(contour_simt_f32(st, wAds, wBds, q, qc, t, ps));
                     step_sums = ps.sums;
                     fused = step_phi = any_phi();
                     stepped = true;

@@ -122,3 +122,30 @@ def test_iterations_equal_oracle(gpu, kind, N, fA, ds):
     q0, q1 = run.get_contour(0, 1), run.get_contour(0, 2)
     step = w * np.asarray(S.diffusion((w * q0).reshape(S.grid_phy))).ravel()
     assert np.abs(q1 - step).max() <= 1e-13 * np.abs(step).max() * 10
+
+
+# FP32 steps of grids off the tensor-core sizes: the triplets of the per-axis passes, bit for bit
+# (batch form 3 runs those), at sides around the 4 x 4 results of a thread, unequal and tiny
+@pytest.mark.parametrize("kind,N", [("P1", (45, 45, 45)), ("P1", (64, 63, 1)), ("P1", (7, 9, 5)), ("PMMM", (34, 62, 18)),
+                                    ("3M", (36, 50, 30)), ("P1", (3, 64, 33))])
+def test_fp32_steps_equal_the_passes(gpu, kind, N):
+    from crysscft_sample_b200 import batch
+
+    rng = np.random.default_rng(4)
+    inst = [{"N": N, "L": (4.2, 4.2, 4.2), "fA": 0.3, "xN": 18.0}]
+    B = batch.BatchSCFT(kind, inst, ds=0.06, precision="fp32")
+    a, b = rng.standard_normal(B.M[0]), rng.standard_normal(B.M[0])
+    B.configure(1, 3)
+    B.set_fields(0, a, b)
+    want = B.iterate(1)["F"][0, 0]
+    G = solvers.make_solver(kind, N)
+    G.set_cell_para((4.2, 4.2, 4.2))
+    run = scft.DiblockSCFT(G, 0.3, 0.06, 18.0, 0.1)
+    run.set_precision("fp32")
+    run.set_fields(a, b)
+    got = run.iterate(1)
+    assert abs(got["F"][0] - want) <= 1e-12 * abs(want)  # FP64 sums in another order
+    w = B.get_fields(0)
+    for k, v in run.get_fields().items():
+        assert np.abs(v - w[k]).max() <= 1e-12 * (1 + np.abs(w[k]).max())
+    B.close()
