@@ -286,6 +286,10 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
 //     with the other chain's, stored long ago (second half of the contour).  The sums alternate
 //     between two accumulators with the parity of k, because those of phase k - 1 may still be on
 //     their way.
+// The first launch of a contour is not dispatched early: the CTAs of a phase take the SMs that those
+// of the phase before leave least occupied, so a first phase that is spread one CTA an SM stays so,
+// while one that was fitted in beside the tail of another kernel puts two of its CTAs on some SMs,
+// and every phase after it does the same (64^3: 5.9 against 10 us a phase).
 // Per iteration on one B200 against what ran these grids before: 16^3 0.186 ms (persistent kernel
 // 0.331), 32^3 0.28 (0.46), 64^3 1.36 (1.46; P1 1.22 against 1.66), 200 steps of 45^3 P1 1.39 (three
 // passes a step 2.13).  A 64^3 phase takes 5.9 us: 4.3 in the CTA (2.4 of DMMA at the peak rate),

@@ -10,8 +10,16 @@
 //
 // Reductions are deterministic: a fixed grid writes per-block partials, the last
 // block to finish (atomic ticket, no waiting) reduces them in a fixed order.
+//
+// On small grids these kernels are launch latency and reduction barriers, nothing else, so they are
+// launched programmatically (each starts with the wait for the one before it, and the next is
+// dispatched meanwhile), several sums share one pair of barriers (block_sums), and the mixing is in
+// the energy kernel.  The kernels around the contour of a 32^3 Anderson iteration (10 iterates): 110
+// us before, 70 after.
 #pragma once
 #include <cuda_runtime.h>
+
+#include "axis_mma.cuh"
 
 namespace crysscft {
 
@@ -40,32 +48,31 @@ __device__ __forceinline__ double warp_max(double v) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
     return v;
 }
-// block-wide sum / max over kRedThreads threads; result valid in thread 0
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-    v = warp_sum(v);
+// block-wide sums (maxima where max_mask has the bit) of K values over kRedThreads threads; results
+// valid in thread 0.  sh: K x kRedThreads / 32 doubles.
+template <int K>
+__device__ __forceinline__ void block_sums(double (&v)[K], double* sh, unsigned max_mask = 0) {
+    constexpr int W = kRedThreads / 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = (max_mask >> k) & 1 ? warp_max(v[k]) : warp_sum(v[k]);
     __syncthreads();
-    if (lane == 0) sh[w] = v;
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (lane == 0) sh[k * W + w] = v[k];
     __syncthreads();
-    double r = 0.0;
     if (w == 0) {
-        r = lane < (kRedThreads / 32) ? sh[lane] : 0.0;
-        r = warp_sum(r);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const double r = lane < W ? sh[k * W + lane] : 0.0;
+            v[k] = (max_mask >> k) & 1 ? warp_max(r) : warp_sum(r);
+        }
     }
-    return r;
 }
-__device__ __forceinline__ double block_max(double v, double* sh) {
-    v = warp_max(v);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[w] = v;
-    __syncthreads();
-    double r = 0.0;
-    if (w == 0) {
-        r = lane < (kRedThreads / 32) ? sh[lane] : 0.0;
-        r = warp_max(r);
-    }
-    return r;
+__device__ __forceinline__ double block_sum(double v, double* sh) {
+    double x[1] = {v};
+    block_sums(x, sh);
+    return x[0];
 }
 
 // Point order of the contour (slices and Boltzmann factors).  The fields are always in the
@@ -94,6 +101,8 @@ __global__ void prep_kernel(const double* __restrict__ wA, const double* __restr
                             double* __restrict__ ksi, T* __restrict__ wAds, T* __restrict__ wBds,
                             T* __restrict__ q_first, T* __restrict__ qc_last, double xN, double ds,
                             long long M, PointOrder po) {
+    pdl_wait();
+    pdl_launch_dependents();
     const double index = -ds / 2;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M;
          i += (long long)gridDim.x * blockDim.x) {
@@ -111,6 +120,8 @@ template <typename T>
 __global__ void __launch_bounds__(kRedThreads)
 q_reduce_kernel(const T* __restrict__ qc0, long long M, double* __restrict__ partials,
                 IterState* st) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ double sh[kRedThreads / 32];
     __shared__ bool last;
     double s = 0.0;
@@ -175,6 +186,8 @@ template <typename T>
 __global__ void phi_kernel(const T* __restrict__ q, const T* __restrict__ qc, double* __restrict__ phiA,
                            double* __restrict__ phiB, const IterState* st, double fA, long long NsA,
                            long long NsB, long long M, PointOrder po) {
+    pdl_wait();
+    pdl_launch_dependents();
     const double Q = st->Q;
     const double fB = 1 - fA;
     const double cA = fA / (NsA * Q);
@@ -232,6 +245,8 @@ __global__ void phi_fused_finish_kernel(const double* __restrict__ acc, const T*
                                         const T* __restrict__ qc, double* __restrict__ phiA,
                                         double* __restrict__ phiB, const IterState* st, double fA, long long NsA,
                                         long long NsB, int n, PointOrder po) {
+    pdl_wait();
+    pdl_launch_dependents();
     const long long n2 = (long long)n * n, M = n2 * n, U = NsA + NsB;
     const double Q = st->Q;
     const double cA = fA / (NsA * Q), cB = (1 - fA) / (NsB * Q);
@@ -276,6 +291,8 @@ template <typename T>
 __global__ void phi_step_finish_kernel(const T* __restrict__ q, const T* __restrict__ qc,
                                        double* __restrict__ phiA, double* __restrict__ phiB, const IterState* st,
                                        double fA, long long NsA, long long NsB, long long M, PhiSlots sp, PointOrder po) {
+    pdl_wait();
+    pdl_launch_dependents();
     const long long U = NsA + NsB;
     const double Q = st->Q;
     const double cA = fA / (NsA * Q), cB = (1 - fA) / (NsB * Q);
@@ -298,37 +315,38 @@ __global__ void phi_step_finish_kernel(const T* __restrict__ q, const T* __restr
     }
 }
 
+// mix: calc_new_fields with acceptance acc in the same pass (simple mixing); else the fields are left
+// to the Anderson kernels, which count the iteration.
 __global__ void __launch_bounds__(kRedThreads)
-energy_kernel(const double* __restrict__ wA, const double* __restrict__ wB,
+energy_kernel(double* __restrict__ wA, double* __restrict__ wB,
               const double* __restrict__ phiA, const double* __restrict__ phiB,
               const double* __restrict__ ksi, double xN, long long M, double* __restrict__ partials,
-              IterState* st, double* __restrict__ hist, unsigned hist_cap) {
-    __shared__ double sh[kRedThreads / 32];
+              IterState* st, double* __restrict__ hist, unsigned hist_cap, int mix, double acc) {
+    __shared__ double sh[5 * (kRedThreads / 32)];
     __shared__ bool last;
-    double e1 = 0.0, eh = 0.0, ek = 0.0, mx = 0.0, rr = 0.0;
+    pdl_wait();
+    pdl_launch_dependents();
+    double s[5] = {0.0, 0.0, 0.0, 0.0, 0.0};  // e1, eh, ek, max incompressibility, |r|^2
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M;
          i += (long long)gridDim.x * blockDim.x) {
         const double pa = phiA[i], pb = phiB[i];
         const double a = wA[i], b = wB[i], x = ksi[i];
-        e1 += -a * pa - b * pb;
-        eh += xN * pa * pb;
+        s[0] += -a * pa - b * pb;
+        s[1] += xN * pa * pb;
         const double temp = 1 - pa - pb;
-        ek += -x * temp;
-        mx = fmax(mx, fabs(temp));
+        s[2] += -x * temp;
+        s[3] = fmax(s[3], fabs(temp));
         const double ra = xN * pb + x - a, rb = xN * pa + x - b;
-        rr += ra * ra + rb * rb;
+        s[4] += ra * ra + rb * rb;
+        if (mix) {
+            wA[i] = a + acc * ra;
+            wB[i] = b + acc * rb;
+        }
     }
-    e1 = block_sum(e1, sh);
-    eh = block_sum(eh, sh);
-    ek = block_sum(ek, sh);
-    mx = block_max(mx, sh);
-    rr = block_sum(rr, sh);
+    block_sums(s, sh, 8u);
     if (threadIdx.x == 0) {
-        partials[5 * blockIdx.x + 0] = e1;
-        partials[5 * blockIdx.x + 1] = eh;
-        partials[5 * blockIdx.x + 2] = ek;
-        partials[5 * blockIdx.x + 3] = mx;
-        partials[5 * blockIdx.x + 4] = rr;
+#pragma unroll
+        for (int k = 0; k < 5; ++k) partials[5 * blockIdx.x + k] = s[k];
         __threadfence();
         const unsigned t = atomicAdd(&st->ticket_e, 1u);
         last = (t == gridDim.x - 1);
@@ -336,25 +354,22 @@ energy_kernel(const double* __restrict__ wA, const double* __restrict__ wB,
     __syncthreads();
     if (!last) return;
     __threadfence();
-    double r1 = 0.0, rh = 0.0, rk = 0.0, rm = 0.0, rs = 0.0;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) s[k] = 0.0;
     for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) {
-        r1 += __ldcg(&partials[5 * i + 0]);
-        rh += __ldcg(&partials[5 * i + 1]);
-        rk += __ldcg(&partials[5 * i + 2]);
-        rm = fmax(rm, __ldcg(&partials[5 * i + 3]));
-        rs += __ldcg(&partials[5 * i + 4]);
+#pragma unroll
+        for (int k = 0; k < 5; ++k) {
+            const double v = __ldcg(&partials[5 * i + k]);
+            s[k] = k == 3 ? fmax(s[k], v) : s[k] + v;
+        }
     }
-    r1 = block_sum(r1, sh);
-    rh = block_sum(rh, sh);
-    rk = block_sum(rk, sh);
-    rm = block_max(rm, sh);
-    rs = block_sum(rs, sh);
+    block_sums(s, sh, 8u);
     if (threadIdx.x == 0) {
         const double Q = st->Q;
         const double fe_entropic_0 = -log(Q);
-        const double fe_entropic_1 = r1 / (double)M;
-        const double fe_enthalpic = rh / (double)M;
-        const double fe_ksi = rk / (double)M;
+        const double fe_entropic_1 = s[0] / (double)M;
+        const double fe_enthalpic = s[1] / (double)M;
+        const double fe_ksi = s[2] / (double)M;
         const double F = fe_entropic_0 + fe_entropic_1 + fe_enthalpic + fe_ksi;
         if (!isfinite(F)) st->error |= 2;
         double* h = hist + (size_t)(st->iteration % hist_cap) * HIST_STRIDE;
@@ -363,24 +378,13 @@ energy_kernel(const double* __restrict__ wA, const double* __restrict__ wB,
         h[HIST_E0] = fe_entropic_0;
         h[HIST_E1] = fe_entropic_1;
         h[HIST_EK] = fe_ksi;
-        h[HIST_MAXINC] = rm;
+        h[HIST_MAXINC] = s[3];
         h[HIST_Q] = Q;
         h[HIST_FLAGS] = (double)st->error;
-        h[HIST_RES] = sqrt(rs / (2.0 * (double)M));
+        h[HIST_RES] = sqrt(s[4] / (2.0 * (double)M));
         st->ticket_e = 0;
+        if (mix) st->iteration += 1;
     }
-}
-
-__global__ void update_kernel(double* __restrict__ wA, double* __restrict__ wB,
-                              const double* __restrict__ phiA, const double* __restrict__ phiB,
-                              const double* __restrict__ ksi, double xN, double acc, long long M,
-                              IterState* st) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M;
-         i += (long long)gridDim.x * blockDim.x) {
-        wA[i] += acc * (xN * phiB[i] + ksi[i] - wA[i]);
-        wB[i] += acc * (xN * phiA[i] + ksi[i] - wB[i]);
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) st->iteration += 1;
 }
 
 // ---------------------------------------------------------------------------
@@ -405,41 +409,53 @@ struct AndersonState {
     unsigned ticket;
 };
 
-// W[head] <- (wA, wB), R[head] <- residual
-__global__ void anderson_record_kernel(const double* __restrict__ wA, const double* __restrict__ wB,
-                                       const double* __restrict__ phiA, const double* __restrict__ phiB,
-                                       const double* __restrict__ ksi, double xN, long long M,
-                                       double* __restrict__ W, double* __restrict__ R, const AndersonState* as) {
-    const long long base = (long long)as->head * 2 * M;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M;
-         i += (long long)gridDim.x * blockDim.x) {
-        const double a = wA[i], b = wB[i], x = ksi[i];
-        W[base + i] = a;
-        W[base + M + i] = b;
-        R[base + i] = xN * phiB[i] + x - a;
-        R[base + M + i] = xN * phiA[i] + x - b;
-    }
-}
-
+// W[head] <- (wA, wB), R[head] <- residual, and
 // gram[head][s_j] = gram[s_j][head] = <R[head], R[s_j]>, j = 0..count (deterministic:
-// per-block partials, the last block reduces them in block order)
+// per-block partials, the last block reduces them in block order).  kDots products share a pass
+// and its barriers.
+constexpr int kDots = 8;
+
 __global__ void __launch_bounds__(kRedThreads)
-anderson_dots_kernel(const double* __restrict__ R, long long M, int slots, double* __restrict__ partials,
-                     AndersonState* as) {
-    __shared__ double sh[kRedThreads / 32];
+anderson_record_kernel(const double* __restrict__ wA, const double* __restrict__ wB,
+                       const double* __restrict__ phiA, const double* __restrict__ phiB,
+                       const double* __restrict__ ksi, double xN, long long M, double* __restrict__ W,
+                       double* __restrict__ R, int slots, double* __restrict__ partials, AndersonState* as) {
+    __shared__ double sh[kDots * (kRedThreads / 32)];
     __shared__ bool last;
+    pdl_wait();
+    pdl_launch_dependents();
     const int head = as->head, count = as->count;
     const long long n2 = 2 * M;
-    const double* r0 = R + (long long)head * n2;
-    for (int j = 0; j <= count; ++j) {
-        const int sj = (head - j + slots) % slots;
-        const double* rj = R + (long long)sj * n2;
-        double d = 0.0;
+    double* r0 = R + (long long)head * n2;
+    double* w0 = W + (long long)head * n2;
+    for (int j0 = 0; j0 <= count; j0 += kDots) {
+        double d[kDots];
+#pragma unroll
+        for (int k = 0; k < kDots; ++k) d[k] = 0.0;
         for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n2;
-             i += (long long)gridDim.x * blockDim.x)
-            d += r0[i] * rj[i];
-        d = block_sum(d, sh);
-        if (threadIdx.x == 0) partials[(size_t)blockIdx.x * (kAndersonMax + 1) + j] = d;
+             i += (long long)gridDim.x * blockDim.x) {
+            double r;
+            if (j0 == 0) {
+                const bool b = i >= M;
+                const long long m = b ? i - M : i;
+                const double w = b ? wB[m] : wA[m];
+                r = xN * (b ? phiA[m] : phiB[m]) + ksi[m] - w;
+                w0[i] = w;
+                r0[i] = r;
+            } else {
+                r = r0[i];
+            }
+#pragma unroll
+            for (int k = 0; k < kDots; ++k)
+                if (j0 + k <= count)
+                    d[k] += r * (j0 + k == 0 ? r : R[(long long)((head - j0 - k + slots) % slots) * n2 + i]);
+        }
+        block_sums(d, sh);
+        if (threadIdx.x == 0) {
+#pragma unroll
+            for (int k = 0; k < kDots; ++k)
+                if (j0 + k <= count) partials[(size_t)blockIdx.x * (kAndersonMax + 1) + j0 + k] = d[k];
+        }
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -449,83 +465,123 @@ anderson_dots_kernel(const double* __restrict__ R, long long M, int slots, doubl
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int j = 0; j <= count; ++j) {
-        double r = 0.0;
-        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
-            r += __ldcg(&partials[(size_t)b * (kAndersonMax + 1) + j]);
-        r = block_sum(r, sh);
+    for (int j0 = 0; j0 <= count; j0 += kDots) {
+        double d[kDots];
+#pragma unroll
+        for (int k = 0; k < kDots; ++k) d[k] = 0.0;
+        for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) {
+#pragma unroll
+            for (int k = 0; k < kDots; ++k)
+                if (j0 + k <= count) d[k] += __ldcg(&partials[(size_t)b * (kAndersonMax + 1) + j0 + k]);
+        }
+        block_sums(d, sh);
         if (threadIdx.x == 0) {
-            const int sj = (head - j + slots) % slots;
-            as->gram[head * (kAndersonMax + 1) + sj] = r;
-            as->gram[sj * (kAndersonMax + 1) + head] = r;
+#pragma unroll
+            for (int k = 0; k < kDots; ++k)
+                if (j0 + k <= count) {
+                    const int sj = (head - j0 - k + slots) % slots;
+                    as->gram[head * (kAndersonMax + 1) + sj] = d[k];
+                    as->gram[sj * (kAndersonMax + 1) + head] = d[k];
+                }
         }
     }
     if (threadIdx.x == 0) as->ticket = 0;
 }
 
-// One thread: the k x k normal equations by Gaussian elimination with partial pivoting;
-// a pivot below 1e-13 of the largest diagonal entry restarts the history (simple step).
-// Then advances the ring.
-__global__ void anderson_solve_kernel(AndersonState* as, int history) {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+// One block: the k x k normal equations by Gaussian elimination with partial pivoting (the first of
+// equal pivots); a pivot below 1e-13 of the largest diagonal entry restarts the history (simple
+// step).  Then advances the ring.  A row per thread of the first warp, the columns of a row shared
+// by the block's warps: one thread took 18 us for 10 iterates.
+__global__ void __launch_bounds__(kRedThreads) anderson_solve_kernel(AndersonState* as, int history) {
+    pdl_wait();
+    pdl_launch_dependents();
+    constexpr int G = kAndersonMax + 1;
+    __shared__ double U[kAndersonMax][G];  // odd row stride: lanes of a column on distinct banks
+    __shared__ double V[kAndersonMax], f[kAndersonMax], c[kAndersonMax];
+    __shared__ int s[G], piv, singular;
     const int slots = history + 1;
     const int n = as->head, k = as->count;
-    constexpr int G = kAndersonMax + 1;
-    int s[kAndersonMax + 1];
-    for (int j = 0; j <= k; ++j) s[j] = (n - j + slots) % slots;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kRedThreads / 32;
+    if (threadIdx.x <= k) s[threadIdx.x] = (n - (int)threadIdx.x + slots) % slots;
+    if (threadIdx.x == 0) singular = 0;
+    __syncthreads();
     const double* g = as->gram;
-    double U[kAndersonMax][kAndersonMax], V[kAndersonMax];
     const double g00 = g[n * G + n];
-    double scale = 0.0;
-    for (int i = 1; i <= k; ++i) {
-        V[i - 1] = g00 - g[n * G + s[i]];
-        for (int j = 1; j <= k; ++j) U[i - 1][j - 1] = g00 - g[n * G + s[j]] - g[s[i] * G + n] + g[s[i] * G + s[j]];
-        scale = fmax(scale, fabs(U[i - 1][i - 1]));
+    for (int e = threadIdx.x; e < k * k; e += kRedThreads) {
+        const int i = e / k, j = e - i * k;
+        U[i][j] = g00 - g[n * G + s[j + 1]] - g[s[i + 1] * G + n] + g[s[i + 1] * G + s[j + 1]];
     }
-    bool singular = false;
-    for (int col = 0; col < k && !singular; ++col) {
-        int piv = col;
-        for (int r = col + 1; r < k; ++r)
-            if (fabs(U[r][col]) > fabs(U[piv][col])) piv = r;
-        if (!(fabs(U[piv][col]) > 1e-13 * scale)) {
-            singular = true;
-            break;
-        }
-        if (piv != col) {
-            for (int j = 0; j < k; ++j) {
-                const double t = U[col][j];
-                U[col][j] = U[piv][j];
-                U[piv][j] = t;
+    if (threadIdx.x < k) V[threadIdx.x] = g00 - g[n * G + s[threadIdx.x + 1]];
+    __syncthreads();
+    double scale = lane < k ? fabs(U[lane][lane]) : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) scale = fmax(scale, __shfl_xor_sync(0xffffffffu, scale, o));
+    for (int col = 0; col < k; ++col) {
+        if (warp == 0) {
+            // largest |U[r][col]|, r >= col, the first of equals
+            double best = lane >= col && lane < k ? fabs(U[lane][col]) : -1.0;
+            int at = lane;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+                if (ob > best || (ob == best && oa < at)) {
+                    best = ob;
+                    at = oa;
+                }
             }
-            const double t = V[col];
-            V[col] = V[piv];
-            V[piv] = t;
+            if (lane == 0) {
+                piv = at;
+                if (!(best > 1e-13 * scale)) singular = 1;
+            }
         }
-        for (int r = col + 1; r < k; ++r) {
-            const double f = U[r][col] / U[col][col];
-            for (int j = col; j < k; ++j) U[r][j] -= f * U[col][j];
-            V[r] -= f * V[col];
+        __syncthreads();
+        if (singular) break;
+        if (piv != col) {
+            if (threadIdx.x < k) {
+                const double x = U[col][threadIdx.x];
+                U[col][threadIdx.x] = U[piv][threadIdx.x];
+                U[piv][threadIdx.x] = x;
+            } else if (threadIdx.x == 32 * (warps - 1)) {
+                const double x = V[col];
+                V[col] = V[piv];
+                V[piv] = x;
+            }
+            __syncthreads();
         }
+        if (warp == 0 && lane > col && lane < k) f[lane] = U[lane][col] / U[col][col];
+        __syncthreads();
+        for (int r = col + 1 + warp; r < k; r += warps) {
+            if (lane >= col && lane < k) U[r][lane] -= f[r] * U[col][lane];
+            if (lane == 0) V[r] -= f[r] * V[col];
+        }
+        __syncthreads();
     }
-    if (!singular) {
+    if (!singular && warp == 0) {
+        double acc = 0.0;  // of row `lane`
         for (int r = k - 1; r >= 0; --r) {
-            double acc = 0.0;
-            for (int j = r + 1; j < k; ++j) acc += U[r][j] * as->c[j];
-            as->c[r] = (V[r] - acc) / U[r][r];
+            if (lane == r) c[r] = (V[r] - acc) / U[r][r];
+            __syncwarp();
+            if (lane < r) acc += U[lane][r] * c[r];
         }
+        if (lane < k) as->c[lane] = c[lane];
     }
-    as->k = singular ? 0 : k;
-    as->restart = singular ? 1 : 0;
-    for (int j = 0; j <= k; ++j) as->slot[j] = s[j];
-    const int kept = singular ? 0 : k;
-    as->count = kept + 1 < history ? kept + 1 : history;
-    as->head = (n + 1) % slots;
+    if (threadIdx.x <= k) as->slot[threadIdx.x] = s[threadIdx.x];
+    if (threadIdx.x == 0) {
+        as->k = singular ? 0 : k;
+        as->restart = singular;
+        const int kept = singular ? 0 : k;
+        as->count = kept + 1 < history ? kept + 1 : history;
+        as->head = (n + 1) % slots;
+    }
 }
 
 // (wA, wB) <- w_0 + sum_j c_j (w_j - w_0) + beta (r_0 + sum_j c_j (r_j - r_0))
 __global__ void anderson_update_kernel(double* __restrict__ wA, double* __restrict__ wB,
                                        const double* __restrict__ W, const double* __restrict__ R,
                                        long long M, const AndersonState* as, double beta, IterState* st) {
+    pdl_wait();
+    pdl_launch_dependents();
     const int k = as->k;
     const long long n2 = 2 * M;
     const double* w0 = W + (long long)as->slot[0] * n2;

@@ -128,6 +128,28 @@ static int upload(void* dst, const void* src, size_t bytes) {
     return SCFT_OK;
 }
 
+// Launch with programmatic stream serialization (unless !early): the kernel may be dispatched while
+// the one before it runs, and waits for it where it says so (pdl_wait).
+template <typename... P, typename... A>
+cudaError_t launch_pdl_if(bool early, void (*fn)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
+                          A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+}
+template <typename... P, typename... A>
+cudaError_t launch_pdl(void (*fn)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+    return launch_pdl_if(true, fn, grid, block, smem, st, std::forward<A>(args)...);
+}
+
 template <typename T>
 struct DevBuf {
     T* p = nullptr;
@@ -915,17 +937,7 @@ struct scft_solver_s {
         CKR(grant_pass((const void*)f, kMmaThreads, smem, &grid));
         const long long lines = row ? p.outer : p.outer * p.inner;
         grid = (int)std::min<long long>(grid, nchain * ((lines + kMmaLines - 1) / kMmaLines));
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)grid);
-        cfg.blockDim = dim3(kMmaThreads);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        CK(cudaLaunchKernelEx(&cfg, f, p));
+        CK(launch_pdl(f, (unsigned)grid, kMmaThreads, smem, st, p));
         ++launches;
         return SCFT_OK;
     }
@@ -983,17 +995,7 @@ struct scft_solver_s {
                 if (a.finish) a.w0[c] = factor(ch[c], k - 1);
                 if (a.start) a.w1[c] = factor(ch[c], k);
             }
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3((unsigned)grid);
-            cfg.blockDim = dim3((unsigned)threads);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = st;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            CK(cudaLaunchKernelEx(&cfg, f, a));
+            CK(launch_pdl(f, (unsigned)grid, (unsigned)threads, smem, st, a));
             ++launches;
         }
         return SCFT_OK;
@@ -1074,17 +1076,8 @@ struct scft_solver_s {
                 if (a.start) a.w1[c] = factor(ch[c], k);
             }
             if (phi) a.phi = phi->of(k);
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3((unsigned)(nchain * std::max(nx, ny)));
-            cfg.blockDim = dim3(kStepThreads);
-            cfg.dynamicSmemBytes = fp.smem;
-            cfg.stream = st;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            CK(cudaLaunchKernelEx(&cfg, fp.fn, a));
+            // the first launch finds the SMs empty (see contour_any_kernel)
+            CK(launch_pdl_if(k > 0, fp.fn, (unsigned)(nchain * std::max(nx, ny)), kStepThreads, fp.smem, st, a));
             ++launches;
         }
         if (phi) phi->finish();
@@ -1623,17 +1616,7 @@ struct scft_diblock_s {
                 if (a.start) a.w1[c] = factor(c, k);
             }
             a.phi = phi.of(k);
-            cudaLaunchConfig_t cfg{};
-            cfg.gridDim = dim3((unsigned)(2 * n));
-            cfg.blockDim = dim3(kContourThreads);
-            cfg.dynamicSmemBytes = step_smem_f32;
-            cfg.stream = st;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            attr[0].val.programmaticStreamSerializationAllowed = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            CK(cudaLaunchKernelEx(&cfg, step_fn_f32, a));
+            CK(launch_pdl_if(k > 0, step_fn_f32, (unsigned)(2 * n), kContourThreads, step_smem_f32, st, a));
             ++solver->launches;
         }
         phi.finish();
@@ -1666,17 +1649,7 @@ struct scft_diblock_s {
                 }
                 // the slab launch of step t - 2, which finished slot t - 1, is two launches back
                 if (half == 0) a.phi = phi.of(t + 1);
-                cudaLaunchConfig_t cfg{};
-                cfg.gridDim = dim3((unsigned)(2 * std::max(nx, ny)));
-                cfg.blockDim = dim3(kSimtThreads);
-                cfg.dynamicSmemBytes = smem;
-                cfg.stream = st;
-                cudaLaunchAttribute attr[1];
-                attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                attr[0].val.programmaticStreamSerializationAllowed = 1;
-                cfg.attrs = attr;
-                cfg.numAttrs = 1;
-                CK(cudaLaunchKernelEx(&cfg, contour_simt_kernel_f32, a));
+                CK(launch_pdl_if(t + half > 0, contour_simt_kernel_f32, (unsigned)(2 * std::max(nx, ny)), kSimtThreads, smem, st, a));
                 ++solver->launches;
             }
         phi.finish();
@@ -1939,6 +1912,10 @@ struct scft_diblock_s {
         size_t launches = 0;
         bool fused = false;  // phi was summed by this iteration's contour kernel
         bool step_phi = false;  // ... of contour_any_kernel, whose sums are
+        // field kernels dispatched early save a launch latency each on small grids; a grid of many
+        // CTAs dispatched beside the tail of another piles up on the SMs that happen to be free
+        // (the phi pass at 64^3: 0.14 -> 0.75 ms)
+        const bool early = MM <= 65536;
         PhiSlots step_sums{};
         PointOrder po{};
         if (sizeof(T) == 8 && solver->ops->pos_order) {
@@ -1948,8 +1925,7 @@ struct scft_diblock_s {
             po.nz = (int)solver->grid_phy[2];
         }
         if (parts & kPartPrep) {
-            prep_kernel<T><<<blocks, 256, 0, st>>>(wA.p, wB.p, ksi.p, wAds, wBds, q, qc + U * M, xN, ds, MM, po);
-            CK(cudaGetLastError());
+            CK(launch_pdl_if(early, prep_kernel<T>, blocks, 256, 0, st, wA.p, wB.p, ksi.p, wAds, wBds, q, qc + U * M, xN, ds, MM, po));
             ++launches;
         }
         if (parts & kPartContour) {
@@ -2024,41 +2000,29 @@ struct scft_diblock_s {
             return SCFT_OK;
         }
         const int rblocks = (int)std::min<long long>(kRedMaxBlocks, (MM + kRedThreads - 1) / kRedThreads);
-        q_reduce_kernel<T><<<rblocks, kRedThreads, 0, st>>>(qc, MM, partials.p, state.p);
-        CK(cudaGetLastError());
+        CK(launch_pdl_if(early, q_reduce_kernel<T>, rblocks, kRedThreads, 0, st, qc, MM, partials.p, state.p));
         if (step_phi)
-            phi_step_finish_kernel<T><<<grid_blocks(MM, 256), 256, 0, st>>>(
-                q, qc, phiA.p, phiB.p, state.p, fA, (long long)NsA, (long long)NsB, MM, step_sums, po);
+            CK(launch_pdl_if(early, phi_step_finish_kernel<T>, grid_blocks(MM, 256), 256, 0, st, q, qc, phiA.p, phiB.p, state.p, fA,
+                          (long long)NsA, (long long)NsB, MM, step_sums, po));
         else if (fused)
-            phi_fused_finish_kernel<T><<<grid_blocks(MM, 256), 256, 0, st>>>(
-                phi_acc.p, q, qc, phiA.p, phiB.p, state.p, fA, (long long)NsA, (long long)NsB,
-                (int)solver->grid_phy[0], po);
+            CK(launch_pdl_if(early, phi_fused_finish_kernel<T>, grid_blocks(MM, 256), 256, 0, st, phi_acc.p, q, qc, phiA.p, phiB.p,
+                          state.p, fA, (long long)NsA, (long long)NsB, (int)solver->grid_phy[0], po));
         else
-            phi_kernel<T><<<grid_blocks((MM + 1) / 2, 256), 256, 0, st>>>(q, qc, phiA.p, phiB.p, state.p, fA,
-                                                                          (long long)NsA, (long long)NsB, MM, po);
-        CK(cudaGetLastError());
+            CK(launch_pdl_if(early, phi_kernel<T>, grid_blocks((MM + 1) / 2, 256), 256, 0, st, q, qc, phiA.p, phiB.p, state.p, fA,
+                          (long long)NsA, (long long)NsB, MM, po));
         if (phase_events) CK(cudaEventRecord(phase_events[3], st));
-        energy_kernel<<<rblocks, kRedThreads, 0, st>>>(wA.p, wB.p, phiA.p, phiB.p, ksi.p, xN, MM,
-                                                       partials.p, state.p, hist.p, hist_cap);
-        CK(cudaGetLastError());
-        if (mix_history > 0) {
-            anderson_record_kernel<<<blocks, 256, 0, st>>>(wA.p, wB.p, phiA.p, phiB.p, ksi.p, xN, MM, and_W.p,
-                                                          and_R.p, and_state.p);
-            CK(cudaGetLastError());
+        const int mix = mix_history > 0 ? 0 : 1;
+        CK(launch_pdl_if(early, energy_kernel, rblocks, kRedThreads, 0, st, wA.p, wB.p, phiA.p, phiB.p, ksi.p, xN, MM, partials.p,
+                      state.p, hist.p, hist_cap, mix, acc));
+        launches += 3;
+        if (!mix) {
             const int dblocks = (int)std::min<long long>(kRedMaxBlocks, (2 * MM + kRedThreads - 1) / kRedThreads);
-            anderson_dots_kernel<<<dblocks, kRedThreads, 0, st>>>(and_R.p, MM, mix_history + 1, and_partials.p,
-                                                                  and_state.p);
-            CK(cudaGetLastError());
-            anderson_solve_kernel<<<1, 32, 0, st>>>(and_state.p, mix_history);
-            CK(cudaGetLastError());
-            anderson_update_kernel<<<grid_blocks(2 * MM, 256), 256, 0, st>>>(wA.p, wB.p, and_W.p, and_R.p, MM,
-                                                                          and_state.p, mix_beta, state.p);
-            CK(cudaGetLastError());
-            launches += 3 + 4;
-        } else {
-            update_kernel<<<blocks, 256, 0, st>>>(wA.p, wB.p, phiA.p, phiB.p, ksi.p, xN, acc, MM, state.p);
-            CK(cudaGetLastError());
-            launches += 4;
+            CK(launch_pdl_if(early, anderson_record_kernel, dblocks, kRedThreads, 0, st, wA.p, wB.p, phiA.p, phiB.p, ksi.p, xN, MM,
+                          and_W.p, and_R.p, mix_history + 1, and_partials.p, and_state.p));
+            CK(launch_pdl_if(early, anderson_solve_kernel, 1, kRedThreads, 0, st, and_state.p, mix_history));
+            CK(launch_pdl_if(early, anderson_update_kernel, grid_blocks(2 * MM, 256), 256, 0, st, wA.p, wB.p, and_W.p, and_R.p, MM,
+                          and_state.p, mix_beta, state.p));
+            launches += 3;
         }
         launches_per_iter = launches;
         return SCFT_OK;
