@@ -37,25 +37,37 @@ static long double gauss(long k, long double L, long double ds) {
     return expl(-ds * kk * kk);
 }
 
-std::vector<long double> pmmm_axis_operator(int n, long double L, long double ds) {
+// A[j][j'] = (1/n) sum_k g_k cos(pi k (2j+1)/2n) cos(pi k (2j'+1)/2n).  A is symmetric and
+// centrosymmetric: a quarter of the entries is summed, the others are their images.
+static std::vector<long double> dct_operator(int n, const std::vector<long double>& g) {
     // cos(pi m / (2n)) for m mod 4n
     const long period = 4L * n;
     std::vector<long double> ctab(period);
     for (long m = 0; m < period; ++m) ctab[m] = cosl(kPi * (long double)m / (2.0L * n));
-    std::vector<long double> g(n);
-    for (int k = 0; k < n; ++k) g[k] = gauss(k, L, ds) * (k == 0 ? 1.0L : 2.0L);
-    std::vector<long double> A((size_t)n * n);
+    std::vector<long double> c((size_t)n * n), gc((size_t)n * n);  // [j][k]
     for (int j = 0; j < n; ++j)
-        for (int jp = 0; jp < n; ++jp) {
+        for (int k = 0; k < n; ++k) {
+            c[(size_t)j * n + k] = ctab[((long)k * (2 * j + 1)) % period];
+            gc[(size_t)j * n + k] = g[k] * c[(size_t)j * n + k];
+        }
+    std::vector<long double> A((size_t)n * n);
+    for (int j = 0; 2 * j < n; ++j)
+        for (int jp = j; jp < n - j; ++jp) {
+            const long double* x = &gc[(size_t)j * n];
+            const long double* y = &c[(size_t)jp * n];
             long double acc = 0.0L;
-            for (int k = 0; k < n; ++k) {
-                long double a = ctab[((long)k * (2 * j + 1)) % period];
-                long double b = ctab[((long)k * (2 * jp + 1)) % period];
-                acc += g[k] * a * b;
-            }
-            A[(size_t)j * n + jp] = acc / (long double)n;
+            for (int k = 0; k < n; ++k) acc += x[k] * y[k];
+            const int mj = n - 1 - j, mp = n - 1 - jp;
+            A[(size_t)j * n + jp] = A[(size_t)jp * n + j] = A[(size_t)mj * n + mp] = A[(size_t)mp * n + mj] =
+                acc / (long double)n;
         }
     return A;
+}
+
+std::vector<long double> pmmm_axis_operator(int n, long double L, long double ds) {
+    std::vector<long double> g(n);
+    for (int k = 0; k < n; ++k) g[k] = gauss(k, L, ds) * (k == 0 ? 1.0L : 2.0L);
+    return dct_operator(n, g);
 }
 
 std::vector<long double> circulant_kernel(int N, long double L, long double ds) {
@@ -108,20 +120,9 @@ static long double dgauss_dL(long k, long double L, long double ds) {
 }
 
 std::vector<long double> pmmm_axis_operator_dL(int n, long double L, long double ds) {
-    const long period = 4L * n;
-    std::vector<long double> ctab(period);
-    for (long m = 0; m < period; ++m) ctab[m] = cosl(kPi * (long double)m / (2.0L * n));
     std::vector<long double> g(n);
     for (int k = 0; k < n; ++k) g[k] = dgauss_dL(k, L, ds) * (k == 0 ? 1.0L : 2.0L);
-    std::vector<long double> A((size_t)n * n);
-    for (int j = 0; j < n; ++j)
-        for (int jp = 0; jp < n; ++jp) {
-            long double acc = 0.0L;
-            for (int k = 0; k < n; ++k)
-                acc += g[k] * ctab[((long)k * (2 * j + 1)) % period] * ctab[((long)k * (2 * jp + 1)) % period];
-            A[(size_t)j * n + jp] = acc / (long double)n;
-        }
-    return A;
+    return dct_operator(n, g);
 }
 
 std::vector<long double> circulant_kernel_dL(int N, long double L, long double ds) {

@@ -177,37 +177,71 @@ struct DevBuf {
     }
 };
 
+// Tables of a set-up that share one device allocation and one upload: placed one by one, then
+// committed.  (A cubic 64^3 set-up has some forty; an allocation and a synchronous copy each took
+// most of the time of a new cell.)
+template <typename T>
+struct Table {
+    T* p = nullptr;
+};
+class TableArena {
+    std::vector<unsigned char> host;
+    std::vector<std::pair<void**, size_t>> slots;
+    DevBuf<unsigned char> dev;
+
+  public:
+    template <typename T, typename S>
+    void place(Table<T>& t, const std::vector<S>& v) {
+        static_assert(sizeof(T) == sizeof(S), "same words");
+        if (v.empty()) return;
+        const size_t off = (host.size() + 255) & ~(size_t)255;
+        host.resize(off + v.size() * sizeof(S));
+        std::memcpy(host.data() + off, v.data(), v.size() * sizeof(S));
+        slots.push_back({reinterpret_cast<void**>(&t.p), off});
+    }
+    int commit() {
+        CKR(dev.alloc(host.size()));
+        CKR(upload(dev.p, host.data(), host.size()));
+        for (auto& s : slots) *s.first = dev.p + s.second;
+        slots.clear();
+        host.clear();
+        host.shrink_to_fit();
+        return SCFT_OK;
+    }
+};
+
 struct OpsSet {
-    DevBuf<double> d_op[3], d_opT[3];
-    DevBuf<float> f_op[3], f_opT[3];
+    TableArena tables, dtables;
+    Table<double> d_op[3], d_opT[3];  // dense operators of axes beyond kMmaMaxN
+    Table<float> f_op[3], f_opT[3];
     // packed per-axis operators for the persistent contour kernel (FP64): for an
     // even/odd axis E then O (h x h, leading dimension h+4), else A (n x n, n+4)
     std::vector<double> h_packed;
-    DevBuf<double> d_packed;
+    Table<double> d_packed;
     // two even/odd levels (PMMM and 3m, n = 64 on every axis): per axis [EE | EO | O]
     // (AxisShapeEO2), x then y then z
     std::vector<double> h_packed2;
-    DevBuf<double> d_packed2;
+    Table<double> d_packed2;
     bool eo2 = false;
     int eo[3] = {0, 0, 0}, off[3] = {0, 0, 0}, ld[3] = {0, 0, 0}, half[3] = {0, 0, 0};
     int total = 0;
     // FP32 precision form: per axis [hi][lo] TF32 split parts, each E,O (even/odd) or A
     std::vector<float> h_packed_f32;
-    DevBuf<float> f_packed;
+    Table<float> f_packed;
     int eo_f32[3] = {0, 0, 0};
     // FP32 precision form on clusters (64-point even/odd axes): per axis the fp16 parts
     // [E_hi | E_lo | O_hi | O_lo] in the tensor cores' K-major operand layout
     std::vector<uint16_t> h_packed_h16;
-    DevBuf<__half> h16_packed;
+    Table<__half> h16_packed;
     int h16_axes = 0;  // axes packed (3: the cluster kernel can run)
     // FFT form of the FP64 axis passes (axis_fft.cuh): per axis the transform length (0: the
     // axis has none), the extension (0 P1, 1 PMMM mirror, 2 3m interleave), the spectrum g
     // (1/NF included) and the NF twiddles
     int fft_nf[3] = {0, 0, 0}, fft_ext[3] = {0, 0, 0};
-    DevBuf<double> d_fft_g[3];
-    DevBuf<double2> d_fft_tw[3];
-    DevBuf<float> f_fft_g[3];   // the same tables rounded to FP32 (precision form)
-    DevBuf<float2> f_fft_tw[3];
+    Table<double> d_fft_g[3];
+    Table<double2> d_fft_tw[3];
+    Table<float> f_fft_g[3];   // the same tables rounded to FP32 (precision form)
+    Table<float2> f_fft_tw[3];
     // FP64 tensor-core axis passes (axis_mma.cuh): the packed blocks of the three axes, one
     // allocation; mode -1: an axis beyond kMmaMaxN
     struct Mma {
@@ -216,7 +250,7 @@ struct OpsSet {
     };
     Mma mma[3], dmma[3];
     Mma one[3];  // axes within kStepMaxN in form kEo1 (contour_any_kernel), in d_mma; mode -1: none
-    DevBuf<double> d_mma, d_dmma;
+    Table<double> d_mma, d_dmma;
     static std::vector<const Mma*> before(const Mma* axes, int ax) {
         std::vector<const Mma*> e;
         for (int a = 0; a < ax; ++a) e.push_back(&axes[a]);
@@ -226,7 +260,7 @@ struct OpsSet {
     // (PointOrder), and the packed FP64 operators of the contour kernels are in that order
     bool pos_order = false;
     // cell-length derivatives dA/dL of the three axis operators (built on first use)
-    DevBuf<double> d_dop[3], d_dopT[3];
+    Table<double> d_dop[3], d_dopT[3];
     bool have_dop = false;
     // an operator that is a sum of Kronecker products (3m with mirror translations):
     // this set holds term 0, `more` the others (their d_op/f_op/d_dop only); the packed
@@ -334,7 +368,7 @@ bool pack_operator_h16(const std::vector<long double>& A, int n, OpsSet& s) {
 // g_k = exp(-ds (2 pi min(k, NF - k) / L)^2) / NF (the factor of K in src/solver_p1.h:149-165,
 // src/solver_Pmmm.h:166-179, src/solver_3m.h:197-231, with the transforms' normalisation),
 // and the twiddles exp(-2 pi i m / NF), both in long double rounded once.
-int upload_fft_tables(OpsSet& s, int axis, int nf, int ext, long double L, long double ds) {
+void place_fft_tables(OpsSet& s, int axis, int nf, int ext, long double L, long double ds) {
     static const long double kPiL = 3.141592653589793238462643383279502884L;
     std::vector<double> g((size_t)nf);
     std::vector<double2> tw((size_t)nf);
@@ -344,23 +378,18 @@ int upload_fft_tables(OpsSet& s, int axis, int nf, int ext, long double L, long 
         const long double a = -2.0L * kPiL * (long double)k / (long double)nf;
         tw[(size_t)k] = make_double2((double)cosl(a), (double)sinl(a));
     }
-    CKR(s.d_fft_g[axis].alloc((size_t)nf));
-    CKR(s.d_fft_tw[axis].alloc((size_t)nf));
-    CKR(upload(s.d_fft_g[axis].p, g.data(), g.size() * sizeof(double)));
-    CKR(upload(s.d_fft_tw[axis].p, tw.data(), tw.size() * sizeof(double2)));
+    s.tables.place(s.d_fft_g[axis], g);
+    s.tables.place(s.d_fft_tw[axis], tw);
     std::vector<float> gf((size_t)nf);
     std::vector<float2> twf((size_t)nf);
     for (int k = 0; k < nf; ++k) {
         gf[(size_t)k] = (float)g[(size_t)k];
         twf[(size_t)k] = make_float2((float)tw[(size_t)k].x, (float)tw[(size_t)k].y);
     }
-    CKR(s.f_fft_g[axis].alloc((size_t)nf));
-    CKR(s.f_fft_tw[axis].alloc((size_t)nf));
-    CKR(upload(s.f_fft_g[axis].p, gf.data(), gf.size() * sizeof(float)));
-    CKR(upload(s.f_fft_tw[axis].p, twf.data(), twf.size() * sizeof(float2)));
+    s.tables.place(s.f_fft_g[axis], gf);
+    s.tables.place(s.f_fft_tw[axis], twf);
     s.fft_nf[axis] = nf;
     s.fft_ext[axis] = ext;
-    return SCFT_OK;
 }
 
 template <typename R>
@@ -550,27 +579,25 @@ void pack_operator_mma(const std::vector<long double>& A0, int n, bool perm, Ops
         }
 }
 
-int upload_operator(const std::vector<long double>& A, int n, OpsSet& s, int axis) {
-    std::vector<double> d((size_t)n * n), dt((size_t)n * n);
-    std::vector<float> f((size_t)n * n), ft((size_t)n * n);
+// Dense copies of one axis operator: FP32 for the SIMT passes, FP64 where no tensor-core pass runs.
+void place_operator(const std::vector<long double>& A, int n, OpsSet& s, int axis) {
+    const size_t nn = (size_t)n * n;
+    const bool fp64 = n > kMmaMaxN;
+    std::vector<double> d(fp64 ? nn : 0), dt(fp64 ? nn : 0);
+    std::vector<float> f(nn), ft(nn);
     for (int i = 0; i < n; ++i)
         for (int j = 0; j < n; ++j) {
             const long double v = A[(size_t)i * n + j];
-            d[(size_t)i * n + j] = (double)v;
-            dt[(size_t)j * n + i] = (double)v;
             f[(size_t)i * n + j] = (float)v;
             ft[(size_t)j * n + i] = (float)v;
+            if (!fp64) continue;
+            d[(size_t)i * n + j] = (double)v;
+            dt[(size_t)j * n + i] = (double)v;
         }
-    const size_t nn = (size_t)n * n;
-    CKR(s.d_op[axis].alloc(nn));
-    CKR(s.d_opT[axis].alloc(nn));
-    CKR(s.f_op[axis].alloc(nn));
-    CKR(s.f_opT[axis].alloc(nn));
-    CKR(upload(s.d_op[axis].p, d.data(), nn * sizeof(double)));
-    CKR(upload(s.d_opT[axis].p, dt.data(), nn * sizeof(double)));
-    CKR(upload(s.f_op[axis].p, f.data(), nn * sizeof(float)));
-    CKR(upload(s.f_opT[axis].p, ft.data(), nn * sizeof(float)));
-    return SCFT_OK;
+    s.tables.place(s.d_op[axis], d);
+    s.tables.place(s.d_opT[axis], dt);
+    s.tables.place(s.f_op[axis], f);
+    s.tables.place(s.f_opT[axis], ft);
 }
 
 int grid_blocks(long long M, int threads) {
@@ -1209,10 +1236,18 @@ struct scft_solver_s {
                               m3sym.par[2] == 0 && m3_no_half_cells();
         s->pos_order = m3_plain && grid_phy[0] <= (size_t)kMmaMaxN && grid_phy[1] <= (size_t)kMmaMaxN &&
                        grid_phy[2] <= (size_t)kMmaMaxN;
+        std::vector<long double> same_axis[3];  // an operator is the same on axes of one length and period
         for (int ax = 0; ax < 3; ++ax) {
-            std::vector<long double> A;
+            std::vector<long double>& A = same_axis[ax];
             const int N = (int)grid_log[ax];
-            if (kind == SCFT_SOLVER_PMMM) {
+            int like = -1;
+            for (int b = 0; b < ax && nt == 1; ++b)
+                if (grid_log[b] == grid_log[ax] && cell[b] == cell[ax] &&
+                    (kind != SCFT_SOLVER_3M || m3sym.par[b] == m3sym.par[ax]))
+                    like = b;
+            if (like >= 0) {
+                A = same_axis[like];
+            } else if (kind == SCFT_SOLVER_PMMM) {
                 A = pmmm_axis_operator(N / 2, (long double)cell[ax], (long double)ds_);
             } else if (kind == SCFT_SOLVER_P1) {
                 A = p1_axis_operator(N, (long double)cell[ax], (long double)ds_);
@@ -1220,13 +1255,13 @@ struct scft_solver_s {
                 const std::vector<long double> c = circulant_kernel(N, (long double)cell[ax], (long double)ds_);
                 for (int t = 1; t < nt; ++t) {
                     const std::vector<long double> B = m3_axis_factor(c, N, m3sym.par[ax], m3terms[(size_t)t][ax]);
-                    CKR(upload_operator(B, (int)grid_phy[ax], *s->term(t), ax));
+                    place_operator(B, (int)grid_phy[ax], *s->term(t), ax);
                     OpsSet* o = s->term(t);
                     pack_operator_mma(B, (int)grid_phy[ax], false, o->mma[ax], h_mma[(size_t)t], OpsSet::before(o->mma, ax));
                 }
                 A = m3_axis_factor(c, N, m3sym.par[ax], m3terms[0][ax]);
             }
-            CKR(upload_operator(A, (int)grid_phy[ax], *s, ax));
+            place_operator(A, (int)grid_phy[ax], *s, ax);
             pack_operator_mma(A, (int)grid_phy[ax], m3_plain, s->mma[ax], h_mma[0], OpsSet::before(s->mma, ax));
             if (nt == 1 && grid_phy[ax] <= (size_t)kStepMaxN)
                 pack_operator_mma(A, (int)grid_phy[ax], m3_plain, s->one[ax], h_mma[0], OpsSet::before(s->one, ax), true);
@@ -1241,29 +1276,19 @@ struct scft_solver_s {
                 else if (m3_plain) { nf = 2 * n; ext = 2; }
                 size_t fsm = 0;
                 if (nf && axis_fft_kernel_for<double>(n, nf, ext, &fsm))
-                    CKR(upload_fft_tables(*s, ax, nf, ext, (long double)cell[ax], (long double)ds_));
+                    place_fft_tables(*s, ax, nf, ext, (long double)cell[ax], (long double)ds_);
             }
             if (kind == SCFT_SOLVER_PMMM && nt == 1) eo2_axes += pack_operator_eo2(A, (int)grid_phy[ax], *s) ? 1 : 0;
             else if (s->pos_order)
                 eo2_axes += pack_operator_eo2(position_order(A, (int)grid_phy[ax]), (int)grid_phy[ax], *s) ? 1 : 0;
         }
-        for (int t = 0; t < nt; ++t) {
-            CKR(s->term(t)->d_mma.alloc(h_mma[(size_t)t].size()));
-            CKR(upload(s->term(t)->d_mma.p, h_mma[(size_t)t].data(), h_mma[(size_t)t].size() * sizeof(double)));
-        }
+        for (int t = 0; t < nt; ++t) s->term(t)->tables.place(s->term(t)->d_mma, h_mma[(size_t)t]);
         s->eo2 = eo2_axes == 3;
-        if (s->eo2) {
-            CKR(s->d_packed2.alloc(s->h_packed2.size()));
-            CKR(upload(s->d_packed2.p, s->h_packed2.data(), s->h_packed2.size() * sizeof(double)));
-        }
-        CKR(s->d_packed.alloc(s->h_packed.size()));
-        CKR(upload(s->d_packed.p, s->h_packed.data(), s->h_packed.size() * sizeof(double)));
-        CKR(s->f_packed.alloc(s->h_packed_f32.size()));
-        CKR(upload(s->f_packed.p, s->h_packed_f32.data(), s->h_packed_f32.size() * sizeof(float)));
-        if (s->h16_axes == 3) {
-            CKR(s->h16_packed.alloc(s->h_packed_h16.size()));
-            CKR(upload(s->h16_packed.p, s->h_packed_h16.data(), s->h_packed_h16.size() * sizeof(uint16_t)));
-        }
+        if (s->eo2) s->tables.place(s->d_packed2, s->h_packed2);
+        s->tables.place(s->d_packed, s->h_packed);
+        s->tables.place(s->f_packed, s->h_packed_f32);
+        if (s->h16_axes == 3) s->tables.place(s->h16_packed, s->h_packed_h16);
+        for (int t = 0; t < nt; ++t) CKR(s->term(t)->tables.commit());
         ops = s.get();
         ops_cache[ds_] = std::move(s);
         ++ops_gen;
@@ -1275,6 +1300,7 @@ struct scft_solver_s {
         if (!ops) return fail(SCFT_ERR_NOT_READY, "set_cell_para/set_contour_step first");
         if (ops->have_dop) return SCFT_OK;
         std::vector<std::vector<double>> h_mma((size_t)ops->nterms);
+        std::vector<long double> same_axis[3];  // term 0 of each axis, as in build_ops
         for (int ax = 0; ax < 3; ++ax) {
             const int N = (int)grid_log[ax];
             const int n = (int)grid_phy[ax];
@@ -1282,31 +1308,39 @@ struct scft_solver_s {
             if (kind == SCFT_SOLVER_3M) dc = circulant_kernel_dL(N, (long double)cell[ax], (long double)ds);
             for (int t = 0; t < ops->nterms; ++t) {
                 std::vector<long double> A;
-                if (kind == SCFT_SOLVER_PMMM)
+                int like = -1;
+                for (int b = 0; b < ax && ops->nterms == 1; ++b)
+                    if (grid_log[b] == grid_log[ax] && cell[b] == cell[ax] &&
+                        (kind != SCFT_SOLVER_3M || m3sym.par[b] == m3sym.par[ax]))
+                        like = b;
+                if (like >= 0)
+                    A = same_axis[like];
+                else if (kind == SCFT_SOLVER_PMMM)
                     A = pmmm_axis_operator_dL(N / 2, (long double)cell[ax], (long double)ds);
                 else if (kind == SCFT_SOLVER_P1)
                     A = p1_axis_operator_dL(N, (long double)cell[ax], (long double)ds);
                 else
                     A = m3_axis_factor(dc, N, m3sym.par[ax], m3terms[(size_t)t][ax]);
-                std::vector<double> d((size_t)n * n), dt((size_t)n * n);
-                for (int i = 0; i < n; ++i)
-                    for (int j = 0; j < n; ++j) {
-                        d[(size_t)i * n + j] = (double)A[(size_t)i * n + j];
-                        dt[(size_t)j * n + i] = (double)A[(size_t)i * n + j];
-                    }
+                if (t == 0) same_axis[ax] = A;
                 OpsSet* o = ops->term(t);
                 // the derivative keeps the operator's symmetry, and so its point order
                 pack_operator_mma(A, n, o->mma[ax].perm != 0, o->dmma[ax], h_mma[(size_t)t], OpsSet::before(o->dmma, ax));
-                CKR(o->d_dop[ax].alloc((size_t)n * n));
-                CKR(o->d_dopT[ax].alloc((size_t)n * n));
-                CKR(upload(o->d_dop[ax].p, d.data(), d.size() * sizeof(double)));
-                CKR(upload(o->d_dopT[ax].p, dt.data(), dt.size() * sizeof(double)));
+                if (n > kMmaMaxN) {
+                    std::vector<double> d((size_t)n * n), dt((size_t)n * n);
+                    for (int i = 0; i < n; ++i)
+                        for (int j = 0; j < n; ++j) {
+                            d[(size_t)i * n + j] = (double)A[(size_t)i * n + j];
+                            dt[(size_t)j * n + i] = (double)A[(size_t)i * n + j];
+                        }
+                    o->dtables.place(o->d_dop[ax], d);
+                    o->dtables.place(o->d_dopT[ax], dt);
+                }
             }
         }
         for (int t = 0; t < ops->nterms; ++t) {
             OpsSet* o = ops->term(t);
-            CKR(o->d_dmma.alloc(h_mma[(size_t)t].size()));
-            CKR(upload(o->d_dmma.p, h_mma[(size_t)t].data(), h_mma[(size_t)t].size() * sizeof(double)));
+            o->dtables.place(o->d_dmma, h_mma[(size_t)t]);
+            CKR(o->dtables.commit());
         }
         ops->have_dop = true;
         return SCFT_OK;
@@ -1475,6 +1509,7 @@ struct scft_diblock_s {
     DevBuf<double> phi_acc;               // its sums: [chain][block][layout][tile][n^2], 8 x space_size_phy
     int last_iter_precision = -1;         // precision of the iteration whose contour is stored
     DevBuf<double> stress_buf;            // batched temporaries of scft_diblock_stress
+    DevBuf<double> stress_part;           // ... and its partial sums
     ContourFnF contour_fn_f32 = nullptr;  // FP32 (3xTF32) contour kernel
     bool cluster_f32 = false;             // FP32 runs on the cluster kernel (contour_cluster_f32.cuh)
     DevBuf<float> f_xch;                  // FP32 exchange buffers
@@ -2609,39 +2644,50 @@ int scft_diblock_stress(scft_diblock_t d, double dlnQ_dL[3], double* dF_dxN, dou
     double* Y = X + tc * M;
     double* T1 = Y + tc * M;
     double* T2 = T1 + tc * M;
+    // one partial per block, axis, term and batch, read back once at the end
+    const long long batches = (U + tc - 1) / tc;
+    const int nterms = s->ops->nterms;
     const int rblocks = (int)std::min<long long>(kRedMaxBlocks, (tc * M + kRedThreads - 1) / kRedThreads);
-    std::vector<double> part(kRedMaxBlocks);
-    for (int ax = 0; ax < 3; ++ax) {
-      double acc = 0.0;
-      // d/dL_a of a sum of Kronecker products: the sum over terms of each term with its
-      // axis-a factor replaced by the derivative factor
-      for (int term = 0; term < s->ops->nterms; ++term) {
-        OpsSet* o = s->ops->term(term);
-        for (int blk = 0; blk < 2; ++blk) {
-            const long long lo = blk == 0 ? 0 : NsA, hi = blk == 0 ? NsA : U;
-            const double* D = blk == 0 ? d->d_wAds.p : d->d_wBds.p;
-            const float* Df = blk == 0 ? d->f_wAds.p : d->f_wBds.p;
-            for (long long t0 = lo; t0 < hi; t0 += tc) {
-                const long long nt = std::min(tc, hi - t0);
+    const size_t rows = (size_t)(3 * nterms) * (size_t)batches;
+    if (d->stress_part.n < rows * (size_t)rblocks) CKR(d->stress_part.alloc(rows * (size_t)rblocks));
+    CK(cudaMemsetAsync(d->stress_part.p, 0, rows * (size_t)rblocks * sizeof(double), st));
+    size_t row = 0;
+    for (long long t0 = 0; t0 < U; t0 += tc) {
+        const long long nt = std::min(tc, U - t0);
+        const int nb = (int)std::min<long long>(rblocks, (nt * M + kRedThreads - 1) / kRedThreads);
+        if (f32)
+            stress_scale_kernel<float><<<grid_blocks(nt * M, 256), 256, 0, st>>>(X, d->f_q.p, d->f_wAds.p, d->f_wBds.p, NsA,
+                                                                                 t0, nt, M);
+        else
+            stress_scale_kernel<double><<<grid_blocks(nt * M, 256), 256, 0, st>>>(X, d->d_q.p, d->d_wAds.p, d->d_wBds.p,
+                                                                                  NsA, t0, nt, M);
+        CK(cudaGetLastError());
+        // d/dL_a of a sum of Kronecker products: the sum over terms of each term with its
+        // axis-a factor replaced by the derivative factor
+        for (int ax = 0; ax < 3; ++ax)
+            for (int term = 0; term < nterms; ++term, ++row) {
+                CKR(s->triplet_batched(X, Y, T1, T2, nt, s->ops->term(term), ax, st, !f32 && s->ops->pos_order));
+                double* part = d->stress_part.p + row * (size_t)rblocks;
                 if (f32)
-                    stress_scale_kernel<float><<<grid_blocks(nt * M, 256), 256, 0, st>>>(X, d->f_q.p, Df, t0, nt, M);
+                    stress_dot_kernel<float><<<nb, kRedThreads, 0, st>>>(d->f_qc.p, d->f_wAds.p, d->f_wBds.p, NsA, Y, t0, nt,
+                                                                         M, part);
                 else
-                    stress_scale_kernel<double><<<grid_blocks(nt * M, 256), 256, 0, st>>>(X, d->d_q.p, D, t0, nt, M);
+                    stress_dot_kernel<double><<<nb, kRedThreads, 0, st>>>(d->d_qc.p, d->d_wAds.p, d->d_wBds.p, NsA, Y, t0,
+                                                                          nt, M, part);
                 CK(cudaGetLastError());
-                CKR(s->triplet_batched(X, Y, T1, T2, nt, o, ax, st, !f32 && s->ops->pos_order));
-                const int nb = (int)std::min<long long>(rblocks, (nt * M + kRedThreads - 1) / kRedThreads);
-                if (f32)
-                    stress_dot_kernel<float><<<nb, kRedThreads, 0, st>>>(d->f_qc.p, Df, Y, t0, nt, M, d->partials.p);
-                else
-                    stress_dot_kernel<double><<<nb, kRedThreads, 0, st>>>(d->d_qc.p, D, Y, t0, nt, M, d->partials.p);
-                CK(cudaGetLastError());
-                CK(cudaMemcpyAsync(part.data(), d->partials.p, nb * sizeof(double), cudaMemcpyDeviceToHost, st));
-                CK(cudaStreamSynchronize(st));
-                for (int i = 0; i < nb; ++i) acc += part[i];
             }
-        }
-      }
-      if (dlnQ_dL) dlnQ_dL[ax] = acc / (double)M / Q;
+    }
+    std::vector<double> part(rows * (size_t)rblocks);
+    CK(cudaMemcpyAsync(part.data(), d->stress_part.p, part.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    for (int ax = 0; ax < 3; ++ax) {
+        double acc = 0.0;
+        for (long long bt = 0; bt < batches; ++bt)
+            for (int term = 0; term < nterms; ++term) {
+                const double* p = part.data() + ((size_t)bt * 3 * nterms + (size_t)(ax * nterms + term)) * (size_t)rblocks;
+                for (int i = 0; i < rblocks; ++i) acc += p[i];
+            }
+        if (dlnQ_dL) dlnQ_dL[ax] = acc / (double)M / Q;
     }
     if (dF_dxN) {
         // F (src/crysSCFT_sample.cpp:404-418) at fixed fields: d(xN <phiA phiB>)/dxN = <phiA phiB>,

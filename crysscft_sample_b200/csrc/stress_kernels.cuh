@@ -11,16 +11,18 @@
 
 namespace crysscft {
 
-// X[i][r] = D[r] * q[(t0 + i) M + r] for i < nt.  T: the stored contour's type (FP32 when
+// X[i][r] = D[r] * q[(t0 + i) M + r] for i < nt, D the Boltzmann factor of segment t0 + i (block A
+// for segments < NsA, else B).  T: the stored contour's type (FP32 when
 // the last iteration ran the precision form); the derivative triplets run in FP64.
 template <typename T>
 __global__ void stress_scale_kernel(double* __restrict__ X, const T* __restrict__ q,
-                                    const T* __restrict__ D, long long t0, long long nt, long long M) {
+                                    const T* __restrict__ DA, const T* __restrict__ DB, long long NsA,
+                                    long long t0, long long nt, long long M) {
     const long long total = nt * M;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
         const long long i = e / M, r = e - i * M;
-        X[e] = (double)D[r] * (double)q[(t0 + i) * M + r];
+        X[e] = (double)(t0 + i < NsA ? DA : DB)[r] * (double)q[(t0 + i) * M + r];
     }
 }
 
@@ -28,15 +30,15 @@ __global__ void stress_scale_kernel(double* __restrict__ X, const T* __restrict_
 // (deterministic: fixed grid, fixed in-block order; the host sums the partials in order)
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads)
-stress_dot_kernel(const T* __restrict__ qc, const T* __restrict__ D, const double* __restrict__ Y,
-                  long long t0, long long nt, long long M, double* __restrict__ partials) {
+stress_dot_kernel(const T* __restrict__ qc, const T* __restrict__ DA, const T* __restrict__ DB, long long NsA,
+                  const double* __restrict__ Y, long long t0, long long nt, long long M, double* __restrict__ partials) {
     __shared__ double sh[kRedThreads / 32];
     const long long total = nt * M;
     double s = 0.0;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
         const long long i = e / M, r = e - i * M;
-        s += (double)qc[(t0 + i + 1) * M + r] * (double)D[r] * Y[e];
+        s += (double)qc[(t0 + i + 1) * M + r] * (double)(t0 + i < NsA ? DA : DB)[r] * Y[e];
     }
     s = block_sum(s, sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = s;
