@@ -291,8 +291,8 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
 // while one that was fitted in beside the tail of another kernel puts two of its CTAs on some SMs,
 // and every phase after it does the same (64^3: 5.9 against 10 us a phase).
 // Per iteration on one B200 against what ran these grids before: 16^3 0.186 ms (persistent kernel
-// 0.331), 32^3 0.28 (0.46), 64^3 1.36 (1.46; P1 1.22 against 1.66), 200 steps of 45^3 P1 1.39 (three
-// passes a step 2.13).  A 64^3 phase takes 5.9 us: 4.3 in the CTA (2.4 of DMMA at the peak rate),
+// 0.331), 24^3 0.34, 32^3 0.26 (0.46), 64^3 1.36 (1.46; P1 1.22 against 1.66), 200 steps of 45^3 P1
+// 1.22 (three passes a step 2.13; 1.40 with run-time trip counts in the K loops).  A 64^3 phase takes 5.9 us: 4.3 in the CTA (2.4 of DMMA at the peak rate),
 // the rest from one launch's last store to the next one's first load.  The same phases as one
 // persistent launch with a release flag per unit pair took 9.1 us (4.5 of them until the last of a
 // CTA's 64 flags was seen), and so did holding back the q stores behind the release.
@@ -326,7 +326,8 @@ struct ContourAnyArgs {
 };
 
 __host__ __device__ inline int step_zpad(int nz) { return (nz + 1) & ~1; }
-__host__ __device__ inline int step_ld(int nz) { return ((nz + 7) & ~7) + 4; }
+// leading dimension of a tile: of the fixed cubic sides their own, else that of the largest
+__host__ __device__ constexpr int step_ld(int side) { return (side ? side : kStepMaxN) + 4; }
 
 // Axis operations of a unit in block form MODE: kEo1 with run-time lengths (NC = 0) or on a cubic
 // grid of side NC; kEo2 / kCirc4 with NC = 64.
@@ -339,40 +340,53 @@ struct StepOp {
     static_assert(G * 2 * VPI <= kStepResults, "results of a lane");
     using Acc = double[ACC][G][1][2];
 
-    template <bool ROW>
-    __device__ __forceinline__ static void run(const double* T, int lf, const double* op, int n, int line0, Acc& acc) {
-        if constexpr (MODE != kEo1) {
-            warp_axis_mma<MODE, NC, 1, ROW>(T, op, line0, acc);
-        } else {
-            const int nn = NC ? NC : n, h = (nn + 1) / 2, hp = (h + 7) & ~7, ld = hp + 4, groups = hp / 8;
-            const int LF = NC ? NC + 4 : lf;
-            const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    // kEo1 with GR groups of 8 pair indices: every trip count known
+    template <bool ROW, int GR>
+    __device__ __forceinline__ static void run_eo1(const double* T, const double* op, int n, int line0, Acc& acc) {
+        constexpr int HP = 8 * GR, LD = HP + 4, LF = step_ld(NC);
+        const int nn = NC ? NC : n, h = (nn + 1) / 2;
+        const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-            for (int r = 0; r < G; ++r)
-                acc[0][r][0][0] = acc[0][r][0][1] = acc[1][r][0][0] = acc[1][r][0][1] = 0.0;
-            const double* f = ROW ? T + (line0 + g) * LF : T + line0 + g;
-            const int KS = ROW ? 1 : LF;
-            const double* B = op + g * ld + t;
-#pragma unroll(NC ? 8 : 2)
-            for (int k0 = 0; k0 < hp; k0 += 4) {
-                const int j = k0 + t, jc = NC || j < h ? j : h - 1;  // padding columns of the operator are 0
-                const double x0 = f[jc * KS], x1 = f[(nn - 1 - jc) * KS];
-                const double u = x0 + x1, v = x0 - x1;
+        for (int r = 0; r < GR; ++r)
+            acc[0][r][0][0] = acc[0][r][0][1] = acc[1][r][0][0] = acc[1][r][0][1] = 0.0;
+        const double* f = ROW ? T + (line0 + g) * LF : T + line0 + g;
+        constexpr int KS = ROW ? 1 : LF;
+        const double* B = op + g * LD + t;
 #pragma unroll
-                for (int r = 0; r < G; ++r) {
-                    if (!NC && r >= groups) continue;
-                    const double e = B[8 * r * ld + k0], o = B[hp * ld + 8 * r * ld + k0];
-                    if (ROW) {
-                        dmma884(acc[0][r][0], u, e);
-                        dmma884(acc[1][r][0], v, o);
-                    } else {
-                        dmma884(acc[0][r][0], e, u);
-                        dmma884(acc[1][r][0], o, v);
-                    }
+        for (int k0 = 0; k0 < HP; k0 += 4) {
+            const int j = k0 + t, jc = NC || j < h ? j : h - 1;  // padding columns of the operator are 0
+            const double x0 = f[jc * KS], x1 = f[(nn - 1 - jc) * KS];
+            const double u = x0 + x1, v = x0 - x1;
+#pragma unroll
+            for (int r = 0; r < GR; ++r) {
+                const double e = B[8 * r * LD + k0], o = B[HP * LD + 8 * r * LD + k0];
+                if (ROW) {
+                    dmma884(acc[0][r][0], u, e);
+                    dmma884(acc[1][r][0], v, o);
+                } else {
+                    dmma884(acc[0][r][0], e, u);
+                    dmma884(acc[1][r][0], o, v);
                 }
             }
         }
     }
+    template <bool ROW>
+    __device__ __forceinline__ static void run(const double* T, const double* op, int n, int line0, Acc& acc) {
+        if constexpr (MODE != kEo1) {
+            warp_axis_mma<MODE, NC, 1, ROW>(T, op, line0, acc);
+        } else if constexpr (NC != 0) {
+            run_eo1<ROW, G>(T, op, n, line0, acc);
+        } else {
+            switch ((n + 15) / 16) {
+                case 1: run_eo1<ROW, 1>(T, op, n, line0, acc); break;
+                case 2: run_eo1<ROW, 2>(T, op, n, line0, acc); break;
+                case 3: run_eo1<ROW, 3>(T, op, n, line0, acc); break;
+                default: run_eo1<ROW, 4>(T, op, n, line0, acc); break;
+            }
+        }
+    }
+    // groups of an axis of n points (kEo1), a bound on those with results
+    __device__ __forceinline__ static bool has_group(int r, int n) { return NC || r < (n + 15) / 16; }
     // results of group r, accumulator element e
     __device__ __forceinline__ static void results(const Acc& acc, int r, int e, double (&y)[VPI]) {
         if constexpr (MODE == kEo1) {
@@ -418,7 +432,8 @@ __global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const Cont
     using Op = StepOp<MODE, NC>;
     constexpr int VPI = Op::VPI, G = Op::G;
     const int nx = NC ? NC : a.n[0], ny = NC ? NC : a.n[1], nz = NC ? NC : a.n[2];
-    const int LF = NC ? NC + 4 : step_ld(nz), zpad = step_zpad(nz);
+    constexpr int LF = step_ld(NC);
+    const int zpad = step_zpad(nz);
     const bool plane = a.plane != 0;
     const int R = plane ? ny : nx;  // rows of the tile; its columns are z
     extern __shared__ __align__(16) double any[];
@@ -475,10 +490,11 @@ __global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const Cont
                 cp_async_wait_all();
             }
             __syncwarp();
-            Op::template run<true>(T, LF, opz, nz, line0, acc);
+            Op::template run<true>(T, opz, nz, line0, acc);
             __syncwarp();
 #pragma unroll
             for (int r4 = 0; r4 < G; ++r4) {
+                if (!Op::has_group(r4, nz)) break;
                 double y0[VPI], y1[VPI];
                 Op::results(acc, r4, 0, y0);
                 Op::results(acc, r4, 1, y1);
@@ -502,12 +518,13 @@ __global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const Cont
         const double* w0 = (c ? a.w0[1] : a.w0[0]) + off;
         const double* w1 = a.start ? (c ? a.w1[1] : a.w1[0]) + off : w0;
         factors(w0);  // in flight during the operation
-        Op::template run<false>(T, LF, opc, R, line0, acc);
+        Op::template run<false>(T, opc, R, line0, acc);
         __syncwarp();
         double* q = (c ? a.q[1] : a.q[0]) + off;
         double v[G * VPI][2];
 #pragma unroll
         for (int r = 0; r < G; ++r) {
+            if (!Op::has_group(r, R)) break;
             double y0[VPI], y1[VPI];
             Op::results(acc, r, 0, y0);
             Op::results(acc, r, 1, y1);
@@ -552,10 +569,11 @@ __global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const Cont
         __syncwarp();
     }
     if (!a.start) return;
-    Op::template run<false>(T, LF, opc, R, line0, acc);
+    Op::template run<false>(T, opc, R, line0, acc);
     double* x = (c ? a.xout[1] : a.xout[0]) + xoff;
 #pragma unroll
     for (int r = 0; r < G; ++r) {
+        if (!Op::has_group(r, R)) break;
         double y0[VPI], y1[VPI];
         Op::results(acc, r, 0, y0);
         Op::results(acc, r, 1, y1);
