@@ -427,40 +427,64 @@ __device__ __forceinline__ void phi_step(const PhiStep<T>& p, long long M) {
     }
 }
 
-template <int MODE, int NC>
-__global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const ContourAnyArgs a) {
-    using Op = StepOp<MODE, NC>;
-    constexpr int VPI = Op::VPI, G = Op::G;
-    const int nx = NC ? NC : a.n[0], ny = NC ? NC : a.n[1], nz = NC ? NC : a.n[2];
-    constexpr int LF = step_ld(NC);
-    const int zpad = step_zpad(nz);
-    const bool plane = a.plane != 0;
-    const int R = plane ? ny : nx;  // rows of the tile; its columns are z
-    extern __shared__ __align__(16) double any[];
-    double* T = any;
-    double* opz = any + ((R + 7) & ~7) * LF;
-    double* opc = a.opc == a.opz ? opz : opz + a.opz_count;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3, line0 = warp * 8;
-    for (int i = threadIdx.x; i < a.opz_count / 2; i += kStepThreads) cp_async16(opz + 2 * i, a.opz + 2 * i);
-    if (opc != opz)
-        for (int i = threadIdx.x; i < a.opc_count / 2; i += kStepThreads) cp_async16(opc + 2 * i, a.opc + 2 * i);
-    cp_async_commit();
-    phi_step(a.phi, (long long)nx * ny * nz);
-    cp_async_wait_all();
-    pdl_wait();
-    pdl_launch_dependents();
-    __syncthreads();  // the operators
+// One unit of one phase: an x-plane or y-slab tile of R rows and nz columns (z) in T.  All pointers
+// are at the unit's first element.
+struct UnitIO {
+    const double* in;   // finish: the exchange buffer of the other layout (row stride xgs); else the initial slice (gs)
+    double* q;          // finish: the finished slice
+    double* x;          // start: this layout's exchange buffer
+    const double* w0;   // finish: Boltzmann factor of the finished step (also in the tile W, see stage_factors)
+    const double* w1;   // start: of the started step (the same pointer within a block)
+    long long gs, xgs;  // row strides of a field and of an exchange buffer
+    int R, nz;
+    bool finish, start, vec;
+    bool active;        // false: this warp has no unit
+};
 
-    const int units = nx > ny ? nx : ny;
-    const int c = (int)blockIdx.x >= units ? 1 : 0, p = (int)blockIdx.x - c * units;
-    if (!NC && p >= (plane ? nx : ny)) return;  // no unit in this layout
-    const long long psz = (long long)ny * nz, xpsz = (long long)ny * zpad;
-    const long long off = plane ? p * psz : (long long)p * nz, gs = plane ? nz : psz;
-    const long long xoff = plane ? p * xpsz : (long long)p * zpad, xgs = plane ? zpad : xpsz;
-    const bool warp_rows = line0 < R, warp_cols = line0 < nz;
+// Copies the factors w (row stride gs) of this warp's rows into the tile W, asynchronously: the
+// caller commits, and contour_unit waits for it with its rows.  The factors are older than the
+// exchange, so their latency passes while a phase waits for its rows; loaded into registers in
+// front of the column operation they held it up (64^3: 2.4 against 1.8 thousand cycles, 16^3 0.7
+// against 0.2).
+template <int NC>
+__device__ __forceinline__ void stage_factors(double* W, const double* w, long long gs, int R_, int nz_, bool vec, int lw) {
+    constexpr int LF = step_ld(NC);
+    const int R = NC ? NC : R_, nz = NC ? NC : nz_;
+    const int lane = threadIdx.x & 31, r = lw * 8 + (lane >> 2), t = lane & 3;
+    if (r >= R) return;
+    if (NC || vec) {
+#pragma unroll(NC ? 8 : 4)
+        for (int ch = t; ch < nz / 2; ch += 4) cp_async16(W + r * LF + 2 * ch, w + r * gs + 2 * ch);
+    } else {
+        for (int z = t; z < nz; z += 4) cp_async8(W + r * LF + z, w + r * gs + z);
+    }
+}
+
+// Copies this warp's rows of the exchange buffer (row stride xgs) into the tile T, asynchronously.
+template <int NC>
+__device__ __forceinline__ void stage_rows(double* T, const double* x, long long xgs, int R_, int nz_, int lw) {
+    constexpr int LF = step_ld(NC);
+    const int R = NC ? NC : R_, zpad = step_zpad(NC ? NC : nz_);
+    const int lane = threadIdx.x & 31, r = lw * 8 + (lane >> 2), t = lane & 3;
+    if (r >= R) return;
+#pragma unroll(NC ? 8 : 4)
+    for (int ch = t; ch < zpad / 2; ch += 4) cp_async16(T + r * LF + 2 * ch, x + r * xgs + 2 * ch);
+}
+
+// Called by all threads of the block, warp lw of those that share the unit taking lines 8 lw.. of T.
+// The results are complete, and T free, after a block barrier.
+template <int MODE, int NC>
+__device__ __forceinline__ void contour_unit(double* T, const double* W, const double* opz, const double* opc,
+                                             const UnitIO& u, int lw) {
+    using Op = StepOp<MODE, NC>;
+    constexpr int VPI = Op::VPI, G = Op::G, LF = step_ld(NC);
+    const int R = NC ? NC : u.R, nz = NC ? NC : u.nz, zpad = step_zpad(nz);
+    const long long gs = u.gs, xgs = u.xgs;
+    const int lane = threadIdx.x & 31;
+    const int g = lane >> 2, t = lane & 3, line0 = lw * 8;
+    const bool warp_rows = u.active && line0 < R, warp_cols = u.active && line0 < nz;
     const int col = line0 + 2 * t;  // this lane's columns: col, col + 1
-    const bool vec = NC || a.vec;
+    const bool vec = NC || u.vec;
     auto ld2 = [&](const double* s) {
         if (vec) return __ldcg(reinterpret_cast<const double2*>(s));
         return make_double2(__ldcg(s), col + 1 < nz ? __ldcg(s + 1) : 0.0);
@@ -476,19 +500,13 @@ __global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const Cont
                 f[r * VPI + k] = row >= 0 && col < nz ? ld2(w + row * gs + col) : make_double2(0.0, 0.0);
             }
     };
-    const double* in = c ? a.in[1] : a.in[0];
     typename Op::Acc acc;
-    if (a.finish) {
+    if (u.finish) {
         // this warp's rows, A_z on them
         if (warp_rows) {
-            const int r = line0 + g;
-            if (NC || r < R) {
-                const double* src = in + xoff + r * xgs;
-#pragma unroll(NC ? 8 : 4)
-                for (int ch = t; ch < zpad / 2; ch += 4) cp_async16(T + r * LF + 2 * ch, src + 2 * ch);
-                cp_async_commit();
-                cp_async_wait_all();
-            }
+            stage_rows<NC>(T, u.in, xgs, R, nz, lw);
+            cp_async_commit();
+            cp_async_wait_all();
             __syncwarp();
             Op::template run<true>(T, opz, nz, line0, acc);
             __syncwarp();
@@ -513,14 +531,11 @@ __global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const Cont
                 }
             }
         }
-        __syncthreads();  // every row is through A_z
+        __syncthreads();  // every row is through A_z, the factors are in
         if (!warp_cols) return;
-        const double* w0 = (c ? a.w0[1] : a.w0[0]) + off;
-        const double* w1 = a.start ? (c ? a.w1[1] : a.w1[0]) + off : w0;
-        factors(w0);  // in flight during the operation
         Op::template run<false>(T, opc, R, line0, acc);
         __syncwarp();
-        double* q = (c ? a.q[1] : a.q[0]) + off;
+        const bool same_w = u.w1 == u.w0;
         double v[G * VPI][2];
 #pragma unroll
         for (int r = 0; r < G; ++r) {
@@ -531,46 +546,53 @@ __global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const Cont
 #pragma unroll
             for (int k = 0; k < VPI; ++k) {
                 const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
-                v[id][0] = y0[k] * f[id].x;
-                v[id][1] = y1[k] * f[id].y;
-                if (row < 0 || col >= nz) continue;
+                if (row < 0) continue;
+                const double2 w = *reinterpret_cast<const double2*>(W + row * LF + col);
+                v[id][0] = y0[k] * w.x;
+                v[id][1] = y1[k] * w.y;
+                if (u.start && same_w)
+                    *reinterpret_cast<double2*>(T + row * LF + col) = make_double2(v[id][0] * w.x, v[id][1] * w.y);
+                if (col >= nz) continue;
                 if (vec) {
-                    __stcg(reinterpret_cast<double2*>(q + row * gs + col), make_double2(v[id][0], v[id][1]));
+                    __stcg(reinterpret_cast<double2*>(u.q + row * gs + col), make_double2(v[id][0], v[id][1]));
                 } else {
-                    __stcg(q + row * gs + col, v[id][0]);
-                    if (col + 1 < nz) __stcg(q + row * gs + col + 1, v[id][1]);
+                    __stcg(u.q + row * gs + col, v[id][0]);
+                    if (col + 1 < nz) __stcg(u.q + row * gs + col + 1, v[id][1]);
                 }
             }
         }
-        if (w1 != w0) factors(w1);  // the step that starts is the first of the other block
+        if (!u.start) return;
+        if (!same_w) {  // the step that starts is the first of the other block
+            factors(u.w1);
 #pragma unroll
-        for (int r = 0; r < G; ++r)
+            for (int r = 0; r < G; ++r) {
+                if (!Op::has_group(r, R)) break;
 #pragma unroll
-            for (int k = 0; k < VPI; ++k) {
-                const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
-                if (row >= 0)
-                    *reinterpret_cast<double2*>(T + row * LF + col) = make_double2(v[id][0] * f[id].x, v[id][1] * f[id].y);
+                for (int k = 0; k < VPI; ++k) {
+                    const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
+                    if (row >= 0)
+                        *reinterpret_cast<double2*>(T + row * LF + col) =
+                            make_double2(v[id][0] * f[id].x, v[id][1] * f[id].y);
+                }
             }
+        }
         __syncwarp();
     } else {
         // the first phase: D q(0), each warp its columns
         if (!warp_cols) return;
-        factors((c ? a.w1[1] : a.w1[0]) + off);
-        const double* src = in + off;
+        factors(u.w1);
 #pragma unroll
         for (int r = 0; r < G; ++r)
 #pragma unroll
             for (int k = 0; k < VPI; ++k) {
                 const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
                 if (row < 0) continue;
-                const double2 x = col < nz ? ld2(src + row * gs + col) : make_double2(0.0, 0.0);
+                const double2 x = col < nz ? ld2(u.in + row * gs + col) : make_double2(0.0, 0.0);
                 *reinterpret_cast<double2*>(T + row * LF + col) = make_double2(x.x * f[id].x, x.y * f[id].y);
             }
         __syncwarp();
     }
-    if (!a.start) return;
     Op::template run<false>(T, opc, R, line0, acc);
-    double* x = (c ? a.xout[1] : a.xout[0]) + xoff;
 #pragma unroll
     for (int r = 0; r < G; ++r) {
         if (!Op::has_group(r, R)) break;
@@ -581,9 +603,55 @@ __global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const Cont
         for (int k = 0; k < VPI; ++k) {
             const int row = Op::position(8 * r + g, k, R);
             if (row >= 0 && col < zpad)  // the padding column takes a dead value
-                __stcg(reinterpret_cast<double2*>(x + row * xgs + col), make_double2(y0[k], y1[k]));
+                __stcg(reinterpret_cast<double2*>(u.x + row * xgs + col), make_double2(y0[k], y1[k]));
         }
     }
+}
+
+template <int MODE, int NC>
+__global__ void __launch_bounds__(kStepThreads, 2) contour_any_kernel(const ContourAnyArgs a) {
+    const int nx = NC ? NC : a.n[0], ny = NC ? NC : a.n[1], nz = NC ? NC : a.n[2];
+    constexpr int LF = step_ld(NC);
+    const int zpad = step_zpad(nz);
+    const bool plane = a.plane != 0;
+    const int R = plane ? ny : nx;  // rows of the tile; its columns are z
+    extern __shared__ __align__(16) double any[];
+    double* T = any;
+    double* W = T + ((R + 7) & ~7) * LF;
+    double* opz = W + ((R + 7) & ~7) * LF;
+    double* opc = a.opc == a.opz ? opz : opz + a.opz_count;
+    const int units = nx > ny ? nx : ny;
+    const int c = (int)blockIdx.x >= units ? 1 : 0, p = (int)blockIdx.x - c * units;
+    const bool has_unit = NC || p < (plane ? nx : ny);  // in this layout
+    const long long psz = (long long)ny * nz, xpsz = (long long)ny * zpad;
+    const long long off = plane ? p * psz : (long long)p * nz, xoff = plane ? p * xpsz : (long long)p * zpad;
+    UnitIO u;
+    u.gs = plane ? nz : psz;
+    u.xgs = plane ? zpad : xpsz;
+    u.in = (c ? a.in[1] : a.in[0]) + (a.finish ? xoff : off);
+    u.q = (c ? a.q[1] : a.q[0]) + off;
+    u.x = (c ? a.xout[1] : a.xout[0]) + xoff;
+    u.w0 = (c ? a.w0[1] : a.w0[0]) + off;
+    u.w1 = (c ? a.w1[1] : a.w1[0]) + off;
+    u.R = R;
+    u.nz = nz;
+    u.finish = a.finish != 0;
+    u.start = a.start != 0;
+    u.vec = a.vec != 0;
+    u.active = true;
+    for (int i = threadIdx.x; i < a.opz_count / 2; i += kStepThreads) cp_async16(opz + 2 * i, a.opz + 2 * i);
+    if (opc != opz)
+        for (int i = threadIdx.x; i < a.opc_count / 2; i += kStepThreads) cp_async16(opc + 2 * i, a.opc + 2 * i);
+    // phase 0 waits for the kernel that writes the factors; they are older than any other launch
+    if (a.finish && has_unit) stage_factors<NC>(W, u.w0, u.gs, R, nz, u.vec, (int)threadIdx.x >> 5);
+    cp_async_commit();
+    phi_step(a.phi, (long long)nx * psz);
+    cp_async_wait_all();
+    pdl_wait();
+    pdl_launch_dependents();
+    __syncthreads();  // the operators
+    if (!has_unit) return;
+    contour_unit<MODE, NC>(T, W, opz, opc, u, (int)threadIdx.x >> 5);
 }
 
 }  // namespace crysscft

@@ -1054,7 +1054,7 @@ struct scft_solver_s {
                        : nx == 16 ? contour_any_kernel<kEo1, 16>
                        : nx == 32 ? contour_any_kernel<kEo1, 32>
                                   : contour_any_kernel<kEo1, 48>);
-        size_t words = (size_t)((std::max(nx, ny) + 7) & ~7) * step_ld(fp.fixed ? nx : 0);
+        size_t words = 2 * (size_t)((std::max(nx, ny) + 7) & ~7) * step_ld(fp.fixed ? nx : 0);  // the tile, its factors
         const size_t cz = (size_t)AxisBlocks(fp.axes[2].mode, nz).count;
         const size_t cy = (size_t)AxisBlocks(fp.axes[1].mode, ny).count, cx = (size_t)AxisBlocks(fp.axes[0].mode, nx).count;
         fp.smem = (words + cz + std::max(cx, cy)) * sizeof(double);
