@@ -1713,7 +1713,7 @@ struct scft_diblock_s {
         }
         if (nx != ny || ny != nz || o->eo_f32[0] != o->eo_f32[1] || o->eo_f32[1] != o->eo_f32[2]) return SCFT_OK;
         // (a caller's own poll limit asks for the kernels that wait)
-        if (force_form == 0 && spin_limit == kSpinLimit && axis_form_override() == 0) {
+        if (force_form <= 1 && spin_limit == kSpinLimit && axis_form_override() == 0) {
             step_fn_f32 = contour_step_kernel_f32_for(nx, o->eo_f32[0], &step_smem_f32);
             if (step_fn_f32) {
                 if (!f_xch.p) CKR(f_xch.alloc(4 * M));
@@ -1813,7 +1813,9 @@ struct scft_diblock_s {
     // wait for the previous launch (16^3 0.186 against 0.202 ms an iteration with the separate
     // pass, 24^3 0.401 / 0.424, 40^3 1.24 / 1.30); on larger grids they reach into the launch they
     // wait for (45^3 1.43 / 1.39, 64^3 1.67 / 1.36 ms).
-    bool any_phi() const { return fused_phi && M <= 65536; }
+    // Not in batch form 1, whose results are those of the batch kernel bit for bit (it leaves phi to
+    // the pass).
+    bool any_phi() const { return fused_phi && M <= 65536 && force_form == 0; }
 
     int setup_persistent() {
         persistent = false;
@@ -1824,7 +1826,7 @@ struct scft_diblock_s {
         if (precision == SCFT_FP32) return setup_persistent_f32();
         any_fp = {};
         // (a caller's own poll limit asks for the kernels that wait)
-        if (force_form == 0 && spin_limit == kSpinLimit) {
+        if (force_form <= 1 && spin_limit == kSpinLimit) {
             CKR(setup_any());
             if (any_fp.fn) return SCFT_OK;
         }
@@ -2933,12 +2935,17 @@ int scft_diblock_time_phases(scft_diblock_t d, size_t n_iter, double out[4]) {
 // ---------------------------------------------------------------------------
 // Planner of the batch kernel (contour_batch.cuh): team sizes and CTA task lists.
 // ---------------------------------------------------------------------------
-// Cost model of one chain on a team of T CTAs (us), fitted to the batch kernel on a B200
-// with every SM busy: per unit and phase 1.9 us of fixed work (tile fetch, waits, barriers,
-// epilogue, stores) plus the axis products, ~1.02e-3 n^2 us; per phase one exchange
-// (release, flag round trip) of ~2.3 us.
-static double team_unit_us(int n) { return 1.9 + 1.02e-3 * (double)n * n; }
-static double team_task_us(int n, int U, int T) { return (U + 1) * ((n / T) * team_unit_us(n) + 2.3); }
+// Cost model of one chain on a team of T CTAs (us), fitted to the batch kernel on a B200 with two
+// CTAs on every SM (sides 16, 24, 32, 48, 64; plans of 4 to 64 instances): per unit and phase 1 us
+// of fixed work (tile fetch, barriers, epilogues, stores) plus the axis products, 2.5e-3 n^2 us, in
+// passes of team_side_by_side(n) units; per phase one exchange (release, flag round trip) of 2 us.
+// A fixed part of 2 us and an exchange of 3 choose other teams (12 instances 3.02 against 2.72 ms an
+// iteration, 64 instances 15.4 / 14.3).
+static double team_unit_us(int n) { return 1.0 + 2.5e-3 * (double)n * n; }
+static double team_task_us(int n, int U, int T) {
+    const int side = n < 8 ? 1 : team_side_by_side(n), units = (n / T + side - 1) / side * side;
+    return (U + 1) * (units * team_unit_us(n) + 2.0);
+}
 
 // First-fit decreasing of durations d into columns of capacity D: the column loads, or
 // an empty vector if one duration exceeds D.  col[i] receives the column of item i.
@@ -3096,7 +3103,7 @@ struct scft_batch_s {
     size_t nstreams = 8;
     int form = 0;
 
-    // Form 4: the contours of every instance whose own plan is the alternating FP64 kernel
+    // Form 4: the contours of every FP64 instance on a cubic grid with a side of 8, 16, .. 64 points
     // run in ONE persistent launch of batch_contour_kernel (contour_batch.cuh); the
     // instances' prep and field kernels stay on the worker streams before and after it.
     std::map<int, int> team_fixed;  // grid side -> team size set by the caller (else the planner's choice)
@@ -3120,28 +3127,41 @@ struct scft_batch_s {
         team_grid = 0;
         struct Ch {
             size_t run;
-            int c, n, U, form;
+            int c, n, U;
         };
         std::vector<Ch> chs;
+        std::vector<scft_solver_s::AnyPlan> plans(n);
         size_t smem = 0;
         for (size_t i = 0; i < n; ++i) {
             scft_diblock_t d = runs[i];
-            if (d->precision != SCFT_FP64 || !d->persistent || !d->alternating || !d->d_q.p || !d->ctrl.p) continue;
-            const int side = (int)d->solver->grid_phy[0];
-            const int f = team_form_for(side, d->solver->ops->eo[0] != 0, d->alt_eo2);
-            if (f < 0) continue;
+            const size_t* g = d->solver->grid_phy;
+            const int side = (int)g[0];
+            if (d->precision != SCFT_FP64 || !d->d_q.p || g[1] != g[0] || g[2] != g[0] || !team_side(side)) continue;
+            plans[i] = d->solver->any_plan(d->solver->ops && d->solver->ops->pos_order);
+            if (!plans[i].fn) continue;
+            if (!d->ctrl.p) {
+                CKR(d->ctrl.alloc(2));
+                CKR(zero_device(d->ctrl.p, 2 * sizeof(unsigned)));
+            }
+            if (d->d_xch.n < 4 * d->M) CKR(d->d_xch.alloc(4 * d->M));
             in_team[i] = 1;
-            smem = std::max(smem, team_form_smem(f));
-            for (int c = 0; c < 2; ++c) chs.push_back(Ch{i, c, side, (int)d->U, f});
+            const OpsSet::Mma* m = plans[i].axes;
+            const int distinct = 1 + (m[1].off != m[2].off) + (m[0].off != m[2].off && m[0].off != m[1].off);
+            smem = std::max(smem, team_smem_bytes(side, distinct, AxisBlocks(m[0].mode, side).count));
+            for (int c = 0; c < 2; ++c) chs.push_back(Ch{i, c, side, (int)d->U});
         }
         if (chs.empty()) return SCFT_OK;
         int sms = 0, dev_smem = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         CK(cudaDeviceGetAttribute(&dev_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
         if (smem > (size_t)dev_smem) return fail(SCFT_ERR_UNSUPPORTED, "batch kernel: shared memory beyond the limit");
-        CK(cudaFuncSetAttribute(batch_contour_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        cudaFuncAttributes fa{};
+        CK(cudaFuncGetAttributes(&fa, (const void*)batch_contour_kernel));
+        // the limit is the function's, shared by every batch: always the device's most
+        CK(cudaFuncSetAttribute(batch_contour_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                dev_smem - (int)fa.sharedSizeBytes));
         int per_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_contour_kernel, kContourThreads, smem));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_contour_kernel, kStepThreads, smem));
         if (per_sm < 1) return fail(SCFT_ERR_UNSUPPORTED, "batch kernel: no block fits on a multiprocessor");
         const int G = per_sm * sms;
 
@@ -3155,7 +3175,7 @@ struct scft_batch_s {
         double planned = 0.0, bound = 0.0;
         CKR(team_schedule(side, steps, G, team_fixed, size, tasks, begin, planned, bound));
 
-        // chain descriptors (tensor maps of each instance's stores and Boltzmann factors)
+        // chain descriptors
         size_t nflags = 0;
         std::vector<size_t> flag_off(chs.size());
         for (size_t j = 0; j < chs.size(); ++j) {
@@ -3170,15 +3190,14 @@ struct scft_batch_s {
             scft_diblock_t d = runs[h.run];
             TeamChain& t = hc[j];
             std::memset(&t, 0, sizeof(TeamChain));
-            double* q = h.c == 0 ? d->d_q.p : d->d_qc.p;
-            for (int v = 0; v < 2; ++v) {  // plane [0] and slab [1] views, as launch_contour
-                CKR(encode_panel_map(&t.tm_q[v], q, h.n, (long long)h.U + 1, v == 0));
-                CKR(encode_panel_map(&t.tm_w[0][v], d->d_wAds.p, h.n, 0, v == 0));
-                CKR(encode_panel_map(&t.tm_w[1][v], d->d_wBds.p, h.n, 0, v == 0));
-            }
-            t.q = q;
+            t.q = h.c == 0 ? d->d_q.p : d->d_qc.p;
+            t.wds[0] = d->d_wAds.p;
+            t.wds[1] = d->d_wBds.p;
             t.xbuf = d->d_xch.p + (size_t)h.c * 2 * d->M;
-            t.ops = d->alt_eo2 ? d->solver->ops->d_packed2.p : d->solver->ops->d_packed.p;
+            const OpsSet::Mma* m = plans[h.run].axes;
+            for (int ax = 0; ax < 3; ++ax) t.op[ax] = d->solver->ops->d_mma.p + m[ax].off;
+            t.op_count = AxisBlocks(m[0].mode, h.n).count;
+            t.mode = m[0].mode;
             t.flags = team_flags.p + flag_off[j];
             t.error = d->ctrl.p + 1;
             t.slot0 = h.c == 0 ? 0 : (long long)h.U;
@@ -3186,7 +3205,6 @@ struct scft_batch_s {
             t.dir = h.c == 0 ? 1 : -1;
             t.U = h.U;
             t.n = h.n;
-            t.form = h.form;
         }
         CKR(team_chains.alloc(hc.size()));
         CKR(team_tasks.alloc(tasks.size()));
@@ -3214,7 +3232,7 @@ struct scft_batch_s {
         for (auto d : runs) a.spin_limit = std::min(a.spin_limit, d->spin_limit);
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)team_grid);
-        cfg.blockDim = dim3(kContourThreads);
+        cfg.blockDim = dim3(kStepThreads);
         cfg.dynamicSmemBytes = team_smem;
         cfg.stream = st;
         cudaLaunchAttribute attr[1];
@@ -3262,7 +3280,7 @@ struct scft_batch_s {
 
     int build_graph() {
         drop_graph();
-        // form 4: the alternating kernel's plan where it applies (the batch kernel runs its schedule)
+        // form 4: the plan of form 1 for the instances that keep their own kernels
         const int ff = form == 4 ? 1 : form;
         for (auto d : runs) {
             d->force_form = ff;

@@ -3,7 +3,7 @@ triplets and chains against the dense per-axis operators, iterations against the
 import numpy as np
 import pytest
 
-from crysscft_sample_b200 import fields, scft, solvers
+from crysscft_sample_b200 import batch, fields, scft, solvers
 from oracle import scft_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -149,3 +149,32 @@ def test_fp32_steps_equal_the_passes(gpu, kind, N):
     for k, v in run.get_fields().items():
         assert np.abs(v - w[k]).max() <= 1e-12 * (1 + np.abs(w[k]).max())
     B.close()
+
+
+# the one-launch batch: every side it takes and block form (reflection, two-level, circulant; equal and
+# different axes; the permuted store of 3M), against one launch per step of each instance, bit for bit
+@pytest.mark.parametrize("teams", [None, {8: 2, 40: 5, 56: 7, 64: 2}])
+@pytest.mark.parametrize("kind,sides,cell", [("PMMM", (8, 40, 56, 64), 4.1), ("3M", (8, 40, 64), list(L)),
+                                             ("P1", (8, 40, 56, 64), list(L)), ("P1", (16, 48, 64), 4.4)])
+def test_batch_sides_equal_step_launches(gpu, kind, sides, cell, teams):
+    m = 1 if kind == "P1" else 2
+    inst = [{"N": (m * s,) * 3, "xN": 16.0 + i, "fA": 0.25 + 0.02 * i, "L": cell, "seed": 7 + i}
+            for i, s in enumerate(sides)]
+    runs = []
+    for form in (1, 4):
+        B = batch.BatchSCFT(kind, inst, ds=0.02)
+        B.configure(4, form)
+        if form == 4:
+            B.set_team_sizes({s: t for s, t in (teams or {}).items() if s in sides})
+        rng = np.random.default_rng(5)
+        for i in range(len(inst)):
+            B.set_fields(i, 16.0 * rng.random(B.M[i]), 16.0 * rng.random(B.M[i]))
+        h = B.iterate(2)
+        if form == 4:
+            assert B.team_plan()["instances"] == len(inst)
+        runs.append((h, [B.get_fields(i) for i in range(len(inst))]))
+        B.close()
+    (h1, f1), (h4, f4) = runs
+    assert np.array_equal(h1["F"], h4["F"]) and np.array_equal(h1["maxinc"], h4["maxinc"])
+    for a, b in zip(f1, f4):
+        assert all(np.array_equal(a[k], b[k]) for k in a)
