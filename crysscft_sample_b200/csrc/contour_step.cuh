@@ -16,10 +16,13 @@
 // starting column operation of a phase need no barrier between them, and one barrier (A_z to
 // columns) is left per tile.  The operator blocks are those of axis_mma.cuh (kEo2, kCirc4).
 //
-// 128^3 PMMM, both chains: 53 us a step against 87 us in three passes (256^3 iteration 17.9 -> 11.6
+// 128^3 PMMM, both chains: 53 us a step against 87 us in three passes (256^3 iteration 17.9 -> 11.5
 // ms), P1 43 against 93 us.  DMMA floor 33 us (P1 22); the rest is the 131 KB that a tile moves in
 // and out four times while its SM computes nothing.  16 warps of 8 lines instead of 8 of 16 at 128
-// points: the same time; at 96 points 12 warps.
+// points: the same time; at 96 points 12 warps.  Turns on the tensor pipe (the two warps of a
+// scheduler one after the other, so that one stores while the other multiplies) gave P1 1.3 % and
+// took 1.8 % from PMMM.  The rows are on their way before the operators have landed: the CTAs of
+// the second wave find no launch to wait for, and had one latency after the other (0.3 to 0.5 %).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -161,10 +164,8 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
     if (opc != opz)
         for (int i = threadIdx.x; i < S::OP / 2; i += S::THREADS) cp_async16(opc + 2 * i, p.opc + 2 * i);
     cp_async_commit();
-    cp_async_wait_all();
     pdl_wait();  // everything above reads only the operators
     pdl_launch_dependents();
-    __syncthreads();
 
     const long long gs = p.plane ? N : (long long)N * N;  // global row stride of a tile
     for (int u = blockIdx.x; u < p.nchain * N; u += gridDim.x) {
@@ -178,6 +179,10 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
             cp_async16(T + r * LF + 2 * ch, in + r * gs + 2 * ch);
         }
         cp_async_commit();
+        if (u == blockIdx.x) {
+            cp_async_wait_but_newest();
+            __syncthreads();  // the operators
+        }
         cp_async_wait_all();
         __syncwarp();
         double acc[4][G][ML][2];
