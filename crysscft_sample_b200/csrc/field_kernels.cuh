@@ -603,12 +603,4 @@ __global__ void anderson_update_kernel(double* __restrict__ wA, double* __restri
     if (blockIdx.x == 0 && threadIdx.x == 0) st->iteration += 1;
 }
 
-// dst[i] = src[i] (type conversion allowed)
-template <typename D, typename S>
-__global__ void convert_kernel(D* __restrict__ dst, const S* __restrict__ src, long long M) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < M;
-         i += (long long)gridDim.x * blockDim.x)
-        dst[i] = (D)src[i];
-}
-
 }  // namespace crysscft

@@ -73,7 +73,7 @@ const char* scft_version(void);
  * N % 4 == 0 on that axis), the component along the mirror normal an even number of
  * grid points; anything else returns SCFT_ERR_INVALID_ARG.  Half-cell components make
  * the triplet a sum of Kronecker products (see scft_operator_terms), which runs on the
- * per-axis kernels instead of the persistent contour kernel.
+ * per-axis kernels instead of the contour kernels.
  * device: CUDA ordinal (-1 = current device). */
 int scft_solver_create(int kind, const size_t grid_size_log[3], const double translational_part[9],
                        int precision, int device, scft_solver_t* out);
@@ -285,10 +285,10 @@ int scft_batch_get_fields(scft_batch_t b, size_t i, double* phiA, double* phiB, 
  * iteration-major. */
 int scft_batch_iterate(scft_batch_t b, size_t n_iter, double* F, double* maxinc);
 /* Worker streams and contour-kernel form (0 automatic, 1 alternating layout, 2 two-phase,
- * 3 per-axis kernels, 4 one persistent launch: the contours of every FP64 instance whose
- * own plan is the alternating kernel run together in one cooperative launch, each chain
+ * 3 per-axis kernels, 4 one persistent launch: the contours of every FP64 instance on a cubic
+ * grid with a side of 8, 16, .. 64 points run together in one cooperative launch, each chain
  * on a team of CTAs that own several x-planes / y-slabs each; the other instances keep
- * their own kernels).  Forms 0-3 launch one contour kernel per instance. */
+ * their own kernels).  Forms 0-3 launch each instance's own contour kernels. */
 int scft_batch_configure(scft_batch_t b, size_t nstreams, int form);
 /* Form 4: fixed team sizes for the listed grid sides (sizes[i] must divide sides[i]);
  * chains of other sides get the planner's choice (scft_team_schedule).  count 0 clears
