@@ -15,10 +15,10 @@
 // Two CTAs share an SM.  A unit is a chain of latencies (fetch, a barrier, three short MMA loops,
 // stores) and a phase ends in a flag round trip, so a second team fills what the first leaves idle.
 // Units of sides below 64 run side by side in a CTA (a warp owns 8 lines, and 8 warps are there).
-// Against one CTA an SM with the next unit's tile prefetched, ms an iteration of the seeded mixture
-// of 8 / 12 / 16 / 24 / 64 instances: 2.46 / 2.72 / 2.48 / 6.04 / 14.3 and 2.8 / 3.3 / 2.86 / 6.4 / 16.2;
-// against one CTA an SM fetching W and X panels by TMA, the kernel before: 2.65 / 3.81 / 2.98 /
-// 7.37 / 15.3.  (4 instances 1.49 / 1.51; 32 of which 11 have 64 points a side 10.2 / 9.9.)
+// ms an iteration of the seeded mixture of 4 / 8 / 12 / 16 / 24 / 32 / 64 instances: 1.38 / 2.34 / 2.52 /
+// 2.39 / 5.59 / 9.37 / 13.2, where one CTA an SM fetching W and X panels by TMA, the kernel before, took
+// 1.51 / 2.65 / 3.81 / 2.98 / 7.37 / 9.86 / 15.3.  One CTA an SM with the next unit's tile prefetched was
+// slower than two (24 instances 6.4 against 6.0, 64 16.2 against 14.3, before contour_unit's last gain).
 //
 // Scheduling: the host (team_schedule in scft.cu) gives every CTA an ordered task list
 // (chain, rank, team size).  CTAs are grouped in columns of one team size; every CTA of a

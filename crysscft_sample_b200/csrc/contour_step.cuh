@@ -295,10 +295,12 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
 // of the phase before leave least occupied, so a first phase that is spread one CTA an SM stays so,
 // while one that was fitted in beside the tail of another kernel puts two of its CTAs on some SMs,
 // and every phase after it does the same (64^3: 5.9 against 10 us a phase).
-// Per iteration on one B200 against what ran these grids before: 16^3 0.186 ms (persistent kernel
-// 0.331), 24^3 0.34, 32^3 0.26 (0.46), 64^3 1.36 (1.46; P1 1.22 against 1.66), 200 steps of 45^3 P1
-// 1.22 (three passes a step 2.13; 1.40 with run-time trip counts in the K loops).  A 64^3 phase takes 5.9 us: 4.3 in the CTA (2.4 of DMMA at the peak rate),
-// the rest from one launch's last store to the next one's first load.  The same phases as one
+// Per iteration on one B200 against what ran these grids before: 16^3 0.173 ms (persistent kernel
+// 0.331), 24^3 0.31, 32^3 0.25 (0.46), 64^3 1.30 (1.46; P1 1.18 against 1.66), 200 steps of 45^3 P1
+// 1.16 (three passes a step 2.13; 1.40 with run-time trip counts in the K loops).  A 64^3 phase takes
+// 5.7 us, 0.55 of it from a launch's last store to the next one's first load.  Of the 9.4 thousand
+// cycles in the CTA 4.6 are DMMA at the peak rate, 1.2 the rows' fetch, 1.3 the epilogue of the
+// finishing operation, the rest latencies and sums around the MMAs.  The same phases as one
 // persistent launch with a release flag per unit pair took 9.1 us (4.5 of them until the last of a
 // CTA's 64 flags was seen), and so did holding back the q stores behind the release.
 // ---------------------------------------------------------------------------
@@ -446,6 +448,21 @@ struct UnitIO {
     bool active;        // false: this warp has no unit
 };
 
+// Copies the 8 rows of warp lw (NC values each, row stride gs) into a tile, asynchronously: 8 lanes
+// on 128 bytes of a row, which fill whole lines and all banks.  (4 lanes a row, as where rows may
+// be short and odd, are two lanes a bank.)
+template <int NC>
+__device__ __forceinline__ void copy_rows(double* tile, const double* x, long long gs, int lw) {
+    const int lane = threadIdx.x & 31, ch = 2 * (lane & 7);
+    if (lw * 8 >= NC) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int r = lw * 8 + 4 * h + (lane >> 3);
+#pragma unroll
+        for (int e = 0; e < NC; e += 16) cp_async16(tile + r * step_ld(NC) + e + ch, x + r * gs + e + ch);
+    }
+}
+
 // Copies the factors w (row stride gs) of this warp's rows into the tile W, asynchronously: the
 // caller commits, and contour_unit waits for it with its rows.  The factors are older than the
 // exchange, so their latency passes while a phase waits for its rows; loaded into registers in
@@ -455,10 +472,14 @@ template <int NC>
 __device__ __forceinline__ void stage_factors(double* W, const double* w, long long gs, int R_, int nz_, bool vec, int lw) {
     constexpr int LF = step_ld(NC);
     const int R = NC ? NC : R_, nz = NC ? NC : nz_;
+    if (NC) {
+        copy_rows<NC>(W, w, gs, lw);
+        return;
+    }
     const int lane = threadIdx.x & 31, r = lw * 8 + (lane >> 2), t = lane & 3;
     if (r >= R) return;
-    if (NC || vec) {
-#pragma unroll(NC ? 8 : 4)
+    if (vec) {
+#pragma unroll 4
         for (int ch = t; ch < nz / 2; ch += 4) cp_async16(W + r * LF + 2 * ch, w + r * gs + 2 * ch);
     } else {
         for (int z = t; z < nz; z += 4) cp_async8(W + r * LF + z, w + r * gs + z);
@@ -469,10 +490,14 @@ __device__ __forceinline__ void stage_factors(double* W, const double* w, long l
 template <int NC>
 __device__ __forceinline__ void stage_rows(double* T, const double* x, long long xgs, int R_, int nz_, int lw) {
     constexpr int LF = step_ld(NC);
-    const int R = NC ? NC : R_, zpad = step_zpad(NC ? NC : nz_);
+    if (NC) {
+        copy_rows<NC>(T, x, xgs, lw);
+        return;
+    }
+    const int R = R_, zpad = step_zpad(nz_);
     const int lane = threadIdx.x & 31, r = lw * 8 + (lane >> 2), t = lane & 3;
     if (r >= R) return;
-#pragma unroll(NC ? 8 : 4)
+#pragma unroll 4
     for (int ch = t; ch < zpad / 2; ch += 4) cp_async16(T + r * LF + 2 * ch, x + r * xgs + 2 * ch);
 }
 
@@ -490,6 +515,15 @@ __device__ __forceinline__ void contour_unit(double* T, const double* W, const d
     const bool warp_rows = u.active && line0 < R, warp_cols = u.active && line0 < nz;
     const int col = line0 + 2 * t;  // this lane's columns: col, col + 1
     const bool vec = NC || u.vec;
+    // The row of this lane's result (r, k) of a column operation.  Rows are 32 bytes past a multiple
+    // of 128, which the operand loads need, so the 16-byte accesses of two neighbouring rows share
+    // banks; lanes of odd g take the mirrored results of a pair in the other order, whose rows lie
+    // 64 bytes apart (NC a multiple of 16).  Shared memory bounds the epilogue: with this and whole
+    // rows in copy_rows a 64^3 PMMM iteration takes 1.302 instead of 1.349 ms, 32^3 0.2535 / 0.2563, 16^3
+    // 0.1733 / 0.1755, a batch of 24 instances 5.6 / 6.0.  (The same exchange in contour_step_kernel:
+    // 256^3 PMMM 11.63 against 11.49 ms.)
+    const bool swap = NC && (g & 1);
+    auto row_of = [&](int r, int k) { return Op::position(8 * r + g, swap ? k ^ 1 : k, R); };
     auto ld2 = [&](const double* s) {
         if (vec) return __ldcg(reinterpret_cast<const double2*>(s));
         return make_double2(__ldcg(s), col + 1 < nz ? __ldcg(s + 1) : 0.0);
@@ -501,7 +535,7 @@ __device__ __forceinline__ void contour_unit(double* T, const double* W, const d
         for (int r = 0; r < G; ++r)
 #pragma unroll
             for (int k = 0; k < VPI; ++k) {
-                const int row = Op::position(8 * r + g, k, R);
+                const int row = row_of(r, k);
                 f[r * VPI + k] = row >= 0 && col < nz ? ld2(w + row * gs + col) : make_double2(0.0, 0.0);
             }
     };
@@ -550,11 +584,11 @@ __device__ __forceinline__ void contour_unit(double* T, const double* W, const d
             Op::results(acc, r, 1, y1);
 #pragma unroll
             for (int k = 0; k < VPI; ++k) {
-                const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
+                const int id = r * VPI + k, row = row_of(r, k);
                 if (row < 0) continue;
                 const double2 w = *reinterpret_cast<const double2*>(W + row * LF + col);
-                v[id][0] = y0[k] * w.x;
-                v[id][1] = y1[k] * w.y;
+                v[id][0] = (swap ? y0[k ^ 1] : y0[k]) * w.x;
+                v[id][1] = (swap ? y1[k ^ 1] : y1[k]) * w.y;
                 if (u.start && same_w)
                     *reinterpret_cast<double2*>(T + row * LF + col) = make_double2(v[id][0] * w.x, v[id][1] * w.y);
                 if (col >= nz) continue;
@@ -574,7 +608,7 @@ __device__ __forceinline__ void contour_unit(double* T, const double* W, const d
                 if (!Op::has_group(r, R)) break;
 #pragma unroll
                 for (int k = 0; k < VPI; ++k) {
-                    const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
+                    const int id = r * VPI + k, row = row_of(r, k);
                     if (row >= 0)
                         *reinterpret_cast<double2*>(T + row * LF + col) =
                             make_double2(v[id][0] * f[id].x, v[id][1] * f[id].y);
@@ -590,7 +624,7 @@ __device__ __forceinline__ void contour_unit(double* T, const double* W, const d
         for (int r = 0; r < G; ++r)
 #pragma unroll
             for (int k = 0; k < VPI; ++k) {
-                const int id = r * VPI + k, row = Op::position(8 * r + g, k, R);
+                const int id = r * VPI + k, row = row_of(r, k);
                 if (row < 0) continue;
                 const double2 x = col < nz ? ld2(u.in + row * gs + col) : make_double2(0.0, 0.0);
                 *reinterpret_cast<double2*>(T + row * LF + col) = make_double2(x.x * f[id].x, x.y * f[id].y);

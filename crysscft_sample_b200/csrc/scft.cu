@@ -2939,7 +2939,7 @@ int scft_diblock_time_phases(scft_diblock_t d, size_t n_iter, double out[4]) {
 // CTAs on every SM (sides 16, 24, 32, 48, 64; plans of 4 to 64 instances): per unit and phase 1 us
 // of fixed work (tile fetch, barriers, epilogues, stores) plus the axis products, 2.5e-3 n^2 us, in
 // passes of team_side_by_side(n) units; per phase one exchange (release, flag round trip) of 2 us.
-// A fixed part of 2 us and an exchange of 3 choose other teams (12 instances 3.02 against 2.72 ms an
+// A fixed part of 2 us and an exchange of 3 chose other teams (12 instances 3.02 against 2.72 ms an
 // iteration, 64 instances 15.4 / 14.3).
 static double team_unit_us(int n) { return 1.0 + 2.5e-3 * (double)n * n; }
 static double team_task_us(int n, int U, int T) {
