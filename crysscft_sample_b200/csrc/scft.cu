@@ -256,9 +256,6 @@ struct OpsSet {
         for (int a = 0; a < ax; ++a) e.push_back(&axes[a]);
         return e;
     }
-    // 3m without translations, axes within kMmaMaxN: the FP64 contour is kept in position order
-    // (PointOrder), and the packed FP64 operators of the contour kernels are in that order
-    bool pos_order = false;
     // cell-length derivatives dA/dL of the three axis operators (built on first use)
     Table<double> d_dop[3], d_dopT[3];
     bool have_dop = false;
@@ -910,6 +907,18 @@ struct scft_solver_s {
     }
 
     int nterms() const { return kind == SCFT_SOLVER_3M ? (int)m3terms.size() : 1; }
+    // 3m without translations: PMMM in another order of the points
+    bool m3_plain() const {
+        return kind == SCFT_SOLVER_3M && nterms() == 1 && m3sym.par[0] == 0 && m3sym.par[1] == 0 &&
+               m3sym.par[2] == 0 && m3_no_half_cells();
+    }
+    // m3_plain, axes within kMmaMaxN: FP64 contours are kept in position order (PointOrder), and the
+    // packed FP64 operators of the contour kernels are in that order.  A property of the solver: a
+    // stored contour keeps it when the operators it came from are gone.
+    bool pos_order() const {
+        return m3_plain() && grid_phy[0] <= (size_t)kMmaMaxN && grid_phy[1] <= (size_t)kMmaMaxN &&
+               grid_phy[2] <= (size_t)kMmaMaxN;
+    }
     bool m3_no_half_cells() const {
         for (int a = 0; a < 3; ++a)
             for (int b = 0; b < 3; ++b)
@@ -978,7 +987,7 @@ struct scft_solver_s {
         if (grid_phy[0] != grid_phy[1] || grid_phy[1] != grid_phy[2]) return 0;
         const OpsSet::Mma* m = o->mma;
         if (m[0].mode != m[1].mode || m[1].mode != m[2].mode) return 0;
-        if (m[0].perm && !o->pos_order) return 0;
+        if (m[0].perm && !pos_order()) return 0;
         size_t smem = 0;
         int th = 0;
         const bool one_op = m[0].off == m[1].off && m[1].off == m[2].off;
@@ -1231,11 +1240,7 @@ struct scft_solver_s {
         for (int t = 1; t < nt; ++t) s->more.push_back(std::make_unique<OpsSet>());
         int eo2_axes = 0;
         std::vector<std::vector<double>> h_mma((size_t)nt);
-        // 3m without translations is PMMM in another order of the points
-        const bool m3_plain = kind == SCFT_SOLVER_3M && nt == 1 && m3sym.par[0] == 0 && m3sym.par[1] == 0 &&
-                              m3sym.par[2] == 0 && m3_no_half_cells();
-        s->pos_order = m3_plain && grid_phy[0] <= (size_t)kMmaMaxN && grid_phy[1] <= (size_t)kMmaMaxN &&
-                       grid_phy[2] <= (size_t)kMmaMaxN;
+        const bool plain = m3_plain(), positions = pos_order();
         std::vector<long double> same_axis[3];  // an operator is the same on axes of one length and period
         for (int ax = 0; ax < 3; ++ax) {
             std::vector<long double>& A = same_axis[ax];
@@ -1262,10 +1267,10 @@ struct scft_solver_s {
                 A = m3_axis_factor(c, N, m3sym.par[ax], m3terms[0][ax]);
             }
             place_operator(A, (int)grid_phy[ax], *s, ax);
-            pack_operator_mma(A, (int)grid_phy[ax], m3_plain, s->mma[ax], h_mma[0], OpsSet::before(s->mma, ax));
+            pack_operator_mma(A, (int)grid_phy[ax], plain, s->mma[ax], h_mma[0], OpsSet::before(s->mma, ax));
             if (nt == 1 && grid_phy[ax] <= (size_t)kStepMaxN)
-                pack_operator_mma(A, (int)grid_phy[ax], m3_plain, s->one[ax], h_mma[0], OpsSet::before(s->one, ax), true);
-            pack_operator(s->pos_order ? position_order(A, (int)grid_phy[ax]) : A, (int)grid_phy[ax], *s, ax);
+                pack_operator_mma(A, (int)grid_phy[ax], plain, s->one[ax], h_mma[0], OpsSet::before(s->one, ax), true);
+            pack_operator(positions ? position_order(A, (int)grid_phy[ax]) : A, (int)grid_phy[ax], *s, ax);
             pack_operator_f32(A, (int)grid_phy[ax], *s, ax);
             if (nt == 1 && s->h16_axes == ax) pack_operator_h16(A, (int)grid_phy[ax], *s);
             {
@@ -1273,13 +1278,13 @@ struct scft_solver_s {
                 int nf = 0, ext = 0;
                 if (kind == SCFT_SOLVER_P1) nf = n;
                 else if (kind == SCFT_SOLVER_PMMM) { nf = 2 * n; ext = 1; }
-                else if (m3_plain) { nf = 2 * n; ext = 2; }
+                else if (plain) { nf = 2 * n; ext = 2; }
                 size_t fsm = 0;
                 if (nf && axis_fft_kernel_for<double>(n, nf, ext, &fsm))
                     place_fft_tables(*s, ax, nf, ext, (long double)cell[ax], (long double)ds_);
             }
             if (kind == SCFT_SOLVER_PMMM && nt == 1) eo2_axes += pack_operator_eo2(A, (int)grid_phy[ax], *s) ? 1 : 0;
-            else if (s->pos_order)
+            else if (positions)
                 eo2_axes += pack_operator_eo2(position_order(A, (int)grid_phy[ax]), (int)grid_phy[ax], *s) ? 1 : 0;
         }
         for (int t = 0; t < nt; ++t) s->term(t)->tables.place(s->term(t)->d_mma, h_mma[(size_t)t]);
@@ -1803,7 +1808,7 @@ struct scft_diblock_s {
 
     // Buffers of an iteration launched step by step (contour_any_kernel), before any capture.
     int setup_any() {
-        any_fp = solver->any_plan(solver->ops && solver->ops->pos_order);
+        any_fp = solver->any_plan(solver->pos_order());
         if (!any_fp.fn) return SCFT_OK;
         if (d_xch.n < 4 * any_fp.x_count) CKR(d_xch.alloc(std::max(4 * M, 4 * any_fp.x_count)));
         if (any_phi() && phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
@@ -1955,7 +1960,7 @@ struct scft_diblock_s {
         const bool early = MM <= 65536;
         PhiSlots step_sums{};
         PointOrder po{};
-        if (sizeof(T) == 8 && solver->ops->pos_order) {
+        if (sizeof(T) == 8 && solver->pos_order()) {
             po.on = 1;
             po.nx = (int)solver->grid_phy[0];
             po.ny = (int)solver->grid_phy[1];
@@ -2668,7 +2673,7 @@ int scft_diblock_stress(scft_diblock_t d, double dlnQ_dL[3], double* dF_dxN, dou
         // axis-a factor replaced by the derivative factor
         for (int ax = 0; ax < 3; ++ax)
             for (int term = 0; term < nterms; ++term, ++row) {
-                CKR(s->triplet_batched(X, Y, T1, T2, nt, s->ops->term(term), ax, st, !f32 && s->ops->pos_order));
+                CKR(s->triplet_batched(X, Y, T1, T2, nt, s->ops->term(term), ax, st, !f32 && s->pos_order()));
                 double* part = d->stress_part.p + row * (size_t)rblocks;
                 if (f32)
                     stress_dot_kernel<float><<<nb, kRedThreads, 0, st>>>(d->f_qc.p, d->f_wAds.p, d->f_wBds.p, NsA, Y, t0, nt,
@@ -2720,7 +2725,7 @@ int scft_diblock_get_contour(scft_diblock_t d, int chain, size_t slot, double* o
     const size_t M = d->M;
     if (d->precision == SCFT_FP64) {
         const double* src = (chain ? d->d_qc.p : d->d_q.p) + slot * M;
-        const bool pos = d->solver->ops && d->solver->ops->pos_order;
+        const bool pos = d->solver->pos_order();
         std::vector<double> tmp(pos ? M : 0);
         CK(cudaMemcpyAsync(pos ? tmp.data() : out, src, M * sizeof(double), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -3137,7 +3142,7 @@ struct scft_batch_s {
             const size_t* g = d->solver->grid_phy;
             const int side = (int)g[0];
             if (d->precision != SCFT_FP64 || !d->d_q.p || g[1] != g[0] || g[2] != g[0] || !team_side(side)) continue;
-            plans[i] = d->solver->any_plan(d->solver->ops && d->solver->ops->pos_order);
+            plans[i] = d->solver->any_plan(d->solver->pos_order());
             if (!plans[i].fn) continue;
             if (!d->ctrl.p) {
                 CKR(d->ctrl.alloc(2));
