@@ -1041,7 +1041,7 @@ struct scft_solver_s {
     // operators, every axis within kStepMaxN points, fields in the point order of the operators.
     struct AnyPlan {
         void (*fn)(const ContourAnyArgs) = nullptr;
-        const OpsSet::Mma* axes = nullptr;
+        OpsSet::Mma axes[3];  // a plan outlives the operators' tables, which it must not point into
         size_t smem = 0;
         size_t x_count = 0;  // doubles of one exchange buffer
         bool fixed = false;  // a cubic side of its own kernel: 16-byte aligned arrays needed
@@ -1056,7 +1056,7 @@ struct scft_solver_s {
         const bool cubic = nx == ny && ny == nz;
         const int m = o->mma[0].mode == o->mma[1].mode && o->mma[1].mode == o->mma[2].mode ? o->mma[0].mode : -1;
         const bool two = cubic && nx == 64 && (m == kEo2 || m == kCirc4);
-        fp.axes = two ? o->mma : o->one;
+        for (int ax = 0; ax < 3; ++ax) fp.axes[ax] = two ? o->mma[ax] : o->one[ax];
         fp.fixed = two || (cubic && (nx == 16 || nx == 32 || nx == 48));
         fp.fn = two ? (m == kEo2 ? contour_any_kernel<kEo2, 64> : contour_any_kernel<kCirc4, 64>)
                     : (!fp.fixed    ? contour_any_kernel<kEo1, 0>
@@ -1560,7 +1560,6 @@ struct scft_diblock_s {
     // FP32 on clusters: 64^3 grids whose three axis operators are centrosymmetric (PMMM,
     // P1), when two 16-CTA clusters with the kernel's shared memory can be resident
     int setup_cluster_f32() {
-        cluster_f32 = false;
         const OpsSet* o = solver->ops;
         if (!o || o->h16_axes != 3 || !o->h16_packed.p || force_form != 0) return SCFT_OK;
         const size_t* g = solver->grid_phy;
@@ -1697,10 +1696,6 @@ struct scft_diblock_s {
     }
 
     int setup_persistent_f32() {
-        persistent = false;
-        f32_phi_fused = false;
-        step_fn_f32 = nullptr;
-        simt_f32 = false;
         CKR(setup_cluster_f32());
         if (cluster_f32) return SCFT_OK;
         const OpsSet* o = solver->ops;
@@ -1823,13 +1818,18 @@ struct scft_diblock_s {
     bool any_phi() const { return fused_phi && M <= 65536 && force_form == 0; }
 
     int setup_persistent() {
+        // nothing of the plan before is left, whichever way this returns
         persistent = false;
         alternating = false;
         alt_eo2 = false;
+        any_fp = {};
+        step_fn_f32 = nullptr;
+        simt_f32 = false;
+        cluster_f32 = false;
+        f32_phi_fused = false;
         if (force_form == 3) return SCFT_OK;  // per-axis kernels only
         if (solver->ops && solver->ops->nterms > 1) return SCFT_OK;  // multi-term: per-axis kernels
         if (precision == SCFT_FP32) return setup_persistent_f32();
-        any_fp = {};
         // (a caller's own poll limit asks for the kernels that wait)
         if (force_form <= 1 && spin_limit == kSpinLimit) {
             CKR(setup_any());

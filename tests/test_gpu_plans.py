@@ -1,8 +1,11 @@
-"""What a launch plan must not outlive: the point order of a stored contour."""
+"""What a launch plan must not outlive: the point order of a stored contour, and the form a batch is
+configured to."""
+import ctypes
+
 import numpy as np
 import pytest
 
-from crysscft_sample_b200 import scft, solvers
+from crysscft_sample_b200 import _lib, batch, scft, solvers
 
 pytestmark = pytest.mark.gpu
 
@@ -28,3 +31,52 @@ def test_a_stored_slice_is_the_same_after_a_new_cell(gpu, kind, N):
     assert np.array_equal(run.get_contour(0, 4), want[1])
     run.close()
     G.close()
+
+
+def _batch(kind, N, precision, first, cell=CELL, U=(0.3, 0.06)):
+    """A batch of one instance that has iterated once in form `first` (None: not at all)."""
+    B = batch.BatchSCFT(kind, [{"N": N, "L": cell, "fA": U[0], "xN": 18.0}], ds=U[1], precision=precision)
+    rng = np.random.default_rng(2)
+    B.w = [rng.standard_normal(B.M[0]) for _ in range(2)]
+    if first is not None:
+        B.configure(1, first)
+        B.set_fields(0, *B.w)
+        B.iterate(1)
+    B.set_fields(0, *B.w)
+    return B
+
+
+# form 3 is the three axis passes a step, whatever ran before it: 4 launches beside 3 a step
+@pytest.mark.parametrize("first", [None, 0, 1, 4])
+@pytest.mark.parametrize("kind,N,precision", [("PMMM", (32, 32, 32), "fp64"), ("P1", (13, 22, 9), "fp64"),
+                                              ("PMMM", (64, 64, 64), "fp32"), ("P1", (13, 22, 9), "fp32")])
+def test_batch_form_3_is_the_axis_passes_after_any_form(gpu, kind, N, precision, first):
+    B, want = _batch(kind, N, precision, first), _batch(kind, N, precision, None)
+    steps = int(0.3 / 0.06) + int(0.7 / 0.06)
+    for b in (B, want):
+        b.configure(1, 3)
+        assert b.launches_per_iteration() == 3 * steps + 4
+    assert np.array_equal(B.iterate(2)["F"], want.iterate(2)["F"])
+    a, b = B.get_fields(0), want.get_fields(0)
+    assert all(np.array_equal(a[k], b[k]) for k in a)
+    B.close()
+    want.close()
+
+
+# a plan keeps nothing of the operators that a new cell frees
+@pytest.mark.parametrize("first", [0, 1, 4])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_batch_form_3_after_a_new_cell(gpu, precision, first):
+    new = (3.7, 4.6, 4.9)
+    B, want = _batch("P1", (13, 22, 9), precision, first), _batch("P1", (13, 22, 9), precision, None, cell=new)
+    B.configure(1, 3)
+    B.iterate(1)
+    lib, d, s = _lib.load(), ctypes.c_void_p(), ctypes.c_void_p()
+    _lib.check(lib.scft_batch_instance(B._h, 0, ctypes.byref(d)))
+    _lib.check(lib.scft_diblock_get_solver(d, ctypes.byref(s)))
+    _lib.check(lib.scft_solver_set_cell_para(s, _lib.dptr(np.array(new + (0.0, 0.0, 0.0)))))
+    B.set_fields(0, *B.w)
+    want.configure(1, 3)
+    assert np.array_equal(B.iterate(2)["F"], want.iterate(2)["F"])
+    B.close()
+    want.close()
