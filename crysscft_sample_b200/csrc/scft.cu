@@ -1705,7 +1705,7 @@ struct scft_diblock_s {
             size_t smem = 0;
             const bool tiled = nx == ny && ny == nz && o->eo_f32[0] == o->eo_f32[1] && o->eo_f32[1] == o->eo_f32[2] &&
                                contour_alt_kernel_f32_for(nx, o->eo_f32[0], &smem) != nullptr;
-            if (!tiled && solver->simt_steps_f32()) {
+            if (!tiled && force_form <= 1 && solver->simt_steps_f32()) {
                 simt_f32 = true;
                 if (any_phi() && phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
                 return SCFT_OK;
@@ -2003,7 +2003,7 @@ struct scft_diblock_s {
                     step_sums = ps.sums;
                     fused = step_phi = any_phi();
                     stepped = true;
-                } else if (!persistent && solver->step_smem()) {
+                } else if (!persistent && force_form <= 1 && solver->step_smem()) {
                     // each chain on a stream of its own: the launches of one chain fill the SMs that
                     // the other's leave (2 x 128 planes on 148 SMs are 1.73 rounds, not 2), and one
                     // chain's loads and stores run under the other's MMAs

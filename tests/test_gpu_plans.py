@@ -80,3 +80,20 @@ def test_batch_form_3_after_a_new_cell(gpu, precision, first):
     assert np.array_equal(B.iterate(2)["F"], want.iterate(2)["F"])
     B.close()
     want.close()
+
+
+# forms 2 and 3 where form 2 has no kernel: cubic 96 and 128, and FP32 off the tensor-core sizes
+@pytest.mark.parametrize("form", [2, 3])
+@pytest.mark.parametrize("kind,N,precision", [("P1", (96, 96, 96), "fp64"), ("PMMM", (256, 256, 256), "fp64"),
+                                              ("P1", (13, 22, 9), "fp32")])
+def test_forms_without_step_launches_keep_the_axis_passes(gpu, kind, N, precision, form):
+    B = _batch(kind, N, precision, None, cell=4.2, U=(0.3, 0.1))
+    B.configure(1, 0)
+    steps = int(0.3 / 0.1) + int(0.7 / 0.1)
+    assert B.launches_per_iteration() < 3 * steps
+    want = B.iterate(1)["F"]
+    B.configure(1, form)
+    assert B.launches_per_iteration() == 3 * steps + 4
+    B.set_fields(0, *B.w)
+    assert np.abs(B.iterate(1)["F"] - want).max() <= 1e-10 * np.abs(want).max()
+    B.close()
