@@ -899,7 +899,6 @@ struct scft_solver_s {
     M3Symmetry m3sym;                 // 3m mirror translations (decoded translational_part)
     std::vector<M3Term> m3terms;      // its Kronecker terms (one when the translations are 0)
     DevBuf<double> d_t3;              // input copy for in-place triplets of multi-term operators
-    DevBuf<double> d_x;               // exchange buffers of chains by contour_any_kernel
 
     ~scft_solver_s() {
         if (iomat) cudaFreeHost(iomat);
@@ -1072,10 +1071,11 @@ struct scft_solver_s {
     }
 
     // U contour steps of nchain chains by contour_any_kernel, one launch per phase; segments < NsA
-    // take w[0], the rest w[1]; x: exchange buffers [layout][chain] of x_count doubles each.
+    // take w[0], the rest w[1]; x: exchange buffers of x_count doubles, one per chain and layout
+    // ([chain], [2 + chain]).
     // phi (two chains over one contour, or null): the sums of q q+ on the way.
     int contour_any(const AnyPlan& fp, int nchain, const ChainSpan* ch, const double* const w[2], long long NsA, size_t U,
-                    double* x, PhiSchedule<double>* phi, cudaStream_t st) {
+                    double* const* x, PhiSchedule<double>* phi, cudaStream_t st) {
         int grid = 1;
         CKR(grant_pass((const void*)fp.fn, kStepThreads, fp.smem, &grid));
         const int nx = (int)grid_phy[0], ny = (int)grid_phy[1], nz = (int)grid_phy[2];
@@ -1105,9 +1105,9 @@ struct scft_solver_s {
             a.opc_count = AxisBlocks(mc.mode, mc.n).count;
             for (int c = 0; c < nchain; ++c) {
                 double* slice = ch[c].q + (ch[c].slot0 + ch[c].dir * k) * M_;
-                a.in[c] = k == 0 ? slice : x + (size_t)((a.plane ? 2 : 0) + c) * fp.x_count;
+                a.in[c] = k == 0 ? slice : x[(a.plane ? 2 : 0) + c];
                 a.q[c] = slice;
-                a.xout[c] = x + (size_t)((a.plane ? 0 : 2) + c) * fp.x_count;
+                a.xout[c] = x[(a.plane ? 0 : 2) + c];
                 if (a.finish) a.w0[c] = factor(ch[c], k - 1);
                 if (a.start) a.w1[c] = factor(ch[c], k);
             }
@@ -1999,7 +1999,9 @@ struct scft_diblock_s {
                     const ChainSpan ch[2] = {{q, 0, 1}, {qc, (long long)U, -1}};
                     const double* w[2] = {wAds, wBds};
                     PhiSchedule<double> ps(q, qc, any_phi() ? phi_acc.p : nullptr, (long long)U, (long long)NsA, MM);
-                    CKR(solver->contour_any(any_fp, 2, ch, w, (long long)NsA, U, d_xch.p, &ps, st));
+                    double* x[4];
+                    for (int i = 0; i < 4; ++i) x[i] = d_xch.p + (size_t)i * any_fp.x_count;
+                    CKR(solver->contour_any(any_fp, 2, ch, w, (long long)NsA, U, x, &ps, st));
                     step_sums = ps.sums;
                     fused = step_phi = any_phi();
                     stepped = true;
@@ -2321,10 +2323,13 @@ static int solver_ready(scft_solver_t s) {
 }
 
 static int ensure_work(scft_solver_t s) {
-    if (s->d_t1.n != s->M) {
+    if (s->d_t2.n == 0) {
+        // t1 and t2 are the exchange buffers of a chain too, whose rows are padded: a chain allocates
+        // nothing that a triplet has not
+        const size_t t = s->grid_phy[0] * s->grid_phy[1] * (size_t)step_zpad((int)s->grid_phy[2]);
         CKR(s->d_io.alloc(s->M));
-        CKR(s->d_t1.alloc(s->M));
-        CKR(s->d_t2.alloc(s->M));
+        CKR(s->d_t1.alloc(t));
+        CKR(s->d_t2.alloc(t));
     }
     if (s->nterms() > 1 && s->d_t3.n != s->M) CKR(s->d_t3.alloc(s->M));
     return SCFT_OK;
@@ -2386,15 +2391,13 @@ int scft_solver_propagate_device(scft_solver_t s, double* d_q, const double* d_i
     const auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
     const ChainSpan ch{d_q, (long long)slot, direction};
     const double* w[2] = {d_wds, d_wds};
+    double* x[4] = {s->d_t1.p, nullptr, s->d_t2.p, nullptr};
     const auto any = s->any_plan(false);
     if (Ns > 0 && any.fn && (!any.fixed || (aligned(d_q) && aligned(d_wds)))) {
-        if (s->d_x.n < 4 * any.x_count) CKR(s->d_x.alloc(4 * any.x_count));
-        return s->contour_any(any, 1, &ch, w, 0, Ns, s->d_x.p, nullptr, st);
+        return s->contour_any(any, 1, &ch, w, 0, Ns, x, nullptr, st);
     }
-    if (Ns > 0 && !s->ops->mma[0].perm && aligned(d_q) && aligned(d_wds) && s->step_smem()) {
-        double* x[4] = {s->d_t1.p, nullptr, s->d_t2.p, nullptr};
+    if (Ns > 0 && !s->ops->mma[0].perm && aligned(d_q) && aligned(d_wds) && s->step_smem())
         return s->contour_steps(1, &ch, w, 0, Ns, x, st);
-    }
     for (size_t k = 0; k < Ns; ++k) {
         const size_t next = direction == 1 ? slot + 1 : slot - 1;
         ChainIO<double> io[2] = {{d_q + slot * M, d_q + next * M, d_wds, d_wds}, {}};

@@ -1,5 +1,5 @@
-"""What a launch plan must not outlive: the point order of a stored contour, and the form a batch is
-configured to."""
+"""What a launch plan must not outlive: the point order of a stored contour, the form a batch was
+configured to, and the buffers a captured call relies on."""
 import ctypes
 
 import numpy as np
@@ -97,3 +97,30 @@ def test_forms_without_step_launches_keep_the_axis_passes(gpu, kind, N, precisio
     B.set_fields(0, *B.w)
     assert np.abs(B.iterate(1)["F"] - want).max() <= 1e-10 * np.abs(want).max()
     B.close()
+
+
+# a chain enqueues and nothing else once a triplet has run: its work buffers are the triplet's
+@pytest.mark.parametrize("kind,n", [("PMMM", (16, 16, 16)), ("P1", (45, 40, 54)), ("P1", (13, 22, 9)), ("P1", (96,) * 3),
+                                    ("3M", (18, 25, 15))])
+def test_a_chain_is_capturable_after_one_triplet(gpu, kind, n):
+    import torch
+
+    G = solvers.make_solver(kind, n if kind == "P1" else tuple(2 * v for v in n))
+    G.set_cell_para(CELL)
+    G.set_contour_step(0.01)
+    M, steps = G.get_space_size_phy(), 5
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    init, w = (torch.rand(M, dtype=torch.float64, device="cuda", generator=gen) for _ in range(2))
+    q = torch.zeros((steps + 1) * M, dtype=torch.float64, device="cuda")
+    G.diffusion_device(init.clone(), torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        G.propagate_device(q, init, w, steps, 1, torch.cuda.current_stream())
+    graph.replay()
+    torch.cuda.synchronize()
+    want = torch.zeros_like(q)
+    G.propagate_device(want, init, w, steps, 1, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    assert torch.equal(q, want)
+    G.close()
