@@ -15,7 +15,8 @@
 // launched programmatically (each starts with the wait for the one before it, and the next is
 // dispatched meanwhile), several sums share one pair of barriers (block_sums), and the mixing is in
 // the energy kernel.  The kernels around the contour of a 32^3 Anderson iteration (10 iterates): 110
-// us before, 70 after.
+// us before, 70 after.  A kernel starts while the one that writes its inputs still runs, so no pointer
+// is __restrict__: that would let the compiler load through it ahead of the wait.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -97,9 +98,9 @@ struct PointOrder {
 };
 
 template <typename T>
-__global__ void prep_kernel(const double* __restrict__ wA, const double* __restrict__ wB,
-                            double* __restrict__ ksi, T* __restrict__ wAds, T* __restrict__ wBds,
-                            T* __restrict__ q_first, T* __restrict__ qc_last, double xN, double ds,
+__global__ void prep_kernel(const double* wA, const double* wB,
+                            double* ksi, T* wAds, T* wBds,
+                            T* q_first, T* qc_last, double xN, double ds,
                             long long M, PointOrder po) {
     pdl_wait();
     pdl_launch_dependents();
@@ -118,7 +119,7 @@ __global__ void prep_kernel(const double* __restrict__ wA, const double* __restr
 
 template <typename T>
 __global__ void __launch_bounds__(kRedThreads)
-q_reduce_kernel(const T* __restrict__ qc0, long long M, double* __restrict__ partials,
+q_reduce_kernel(const T* qc0, long long M, double* partials,
                 IterState* st) {
     pdl_wait();
     pdl_launch_dependents();
@@ -166,7 +167,7 @@ struct Pair<float> {
 };
 
 template <typename T>
-__device__ __forceinline__ void phi_point_pair(const T* __restrict__ q, const T* __restrict__ qc, long long M,
+__device__ __forceinline__ void phi_point_pair(const T* q, const T* qc, long long M,
                                                long long i, long long s0, long long ns, double c, double& a0,
                                                double& a1) {
     using P = typename Pair<T>::type;
@@ -183,8 +184,8 @@ __device__ __forceinline__ void phi_point_pair(const T* __restrict__ q, const T*
 }
 
 template <typename T>
-__global__ void phi_kernel(const T* __restrict__ q, const T* __restrict__ qc, double* __restrict__ phiA,
-                           double* __restrict__ phiB, const IterState* st, double fA, long long NsA,
+__global__ void phi_kernel(const T* q, const T* qc, double* phiA,
+                           double* phiB, const IterState* st, double fA, long long NsA,
                            long long NsB, long long M, PointOrder po) {
     pdl_wait();
     pdl_launch_dependents();
@@ -241,9 +242,9 @@ __global__ void phi_kernel(const T* __restrict__ q, const T* __restrict__ qc, do
 // element of grid point (x, y, z) is (z / 8) * 8n + row * 8 + z % 8, with row y in plane
 // tile x and row x in slab tile y.
 template <typename T>
-__global__ void phi_fused_finish_kernel(const double* __restrict__ acc, const T* __restrict__ q,
-                                        const T* __restrict__ qc, double* __restrict__ phiA,
-                                        double* __restrict__ phiB, const IterState* st, double fA, long long NsA,
+__global__ void phi_fused_finish_kernel(const double* acc, const T* q,
+                                        const T* qc, double* phiA,
+                                        double* phiB, const IterState* st, double fA, long long NsA,
                                         long long NsB, int n, PointOrder po) {
     pdl_wait();
     pdl_launch_dependents();
@@ -288,8 +289,8 @@ struct PhiSlots {
     long long s[8];
 };
 template <typename T>
-__global__ void phi_step_finish_kernel(const T* __restrict__ q, const T* __restrict__ qc,
-                                       double* __restrict__ phiA, double* __restrict__ phiB, const IterState* st,
+__global__ void phi_step_finish_kernel(const T* q, const T* qc,
+                                       double* phiA, double* phiB, const IterState* st,
                                        double fA, long long NsA, long long NsB, long long M, PhiSlots sp, PointOrder po) {
     pdl_wait();
     pdl_launch_dependents();
@@ -318,10 +319,10 @@ __global__ void phi_step_finish_kernel(const T* __restrict__ q, const T* __restr
 // mix: calc_new_fields with acceptance acc in the same pass (simple mixing); else the fields are left
 // to the Anderson kernels, which count the iteration.
 __global__ void __launch_bounds__(kRedThreads)
-energy_kernel(double* __restrict__ wA, double* __restrict__ wB,
-              const double* __restrict__ phiA, const double* __restrict__ phiB,
-              const double* __restrict__ ksi, double xN, long long M, double* __restrict__ partials,
-              IterState* st, double* __restrict__ hist, unsigned hist_cap, int mix, double acc) {
+energy_kernel(double* wA, double* wB,
+              const double* phiA, const double* phiB,
+              const double* ksi, double xN, long long M, double* partials,
+              IterState* st, double* hist, unsigned hist_cap, int mix, double acc) {
     __shared__ double sh[5 * (kRedThreads / 32)];
     __shared__ bool last;
     pdl_wait();
@@ -416,10 +417,10 @@ struct AndersonState {
 constexpr int kDots = 8;
 
 __global__ void __launch_bounds__(kRedThreads)
-anderson_record_kernel(const double* __restrict__ wA, const double* __restrict__ wB,
-                       const double* __restrict__ phiA, const double* __restrict__ phiB,
-                       const double* __restrict__ ksi, double xN, long long M, double* __restrict__ W,
-                       double* __restrict__ R, int slots, double* __restrict__ partials, AndersonState* as) {
+anderson_record_kernel(const double* wA, const double* wB,
+                       const double* phiA, const double* phiB,
+                       const double* ksi, double xN, long long M, double* W,
+                       double* R, int slots, double* partials, AndersonState* as) {
     __shared__ double sh[kDots * (kRedThreads / 32)];
     __shared__ bool last;
     pdl_wait();
@@ -577,8 +578,8 @@ __global__ void __launch_bounds__(kRedThreads) anderson_solve_kernel(AndersonSta
 }
 
 // (wA, wB) <- w_0 + sum_j c_j (w_j - w_0) + beta (r_0 + sum_j c_j (r_j - r_0))
-__global__ void anderson_update_kernel(double* __restrict__ wA, double* __restrict__ wB,
-                                       const double* __restrict__ W, const double* __restrict__ R,
+__global__ void anderson_update_kernel(double* wA, double* wB,
+                                       const double* W, const double* R,
                                        long long M, const AndersonState* as, double beta, IterState* st) {
     pdl_wait();
     pdl_launch_dependents();
