@@ -27,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include "axis_mma.cuh"
+#include "phi_schedule.h"
 
 namespace crysscft {
 
@@ -307,15 +308,6 @@ __global__ void __launch_bounds__(StepShape<MODE, N, ML>::THREADS, 1) contour_st
 constexpr int kStepMaxN = 64;
 constexpr int kStepThreads = 256;
 constexpr int kStepResults = 16;  // results of a lane in one operation
-
-// phi work of one phase: acc += q qc of up to two slots (null pointers: none)
-template <typename T>
-struct PhiStep {
-    const T* q[2];
-    const T* qc[2];
-    double* acc[2];
-    int add[2];  // 0: the first term of this accumulator
-};
 
 struct ContourAnyArgs {
     const double* in[2];   // k = 0: the initial slice; else the exchange buffer of the other layout

@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include "axis_mma.cuh"
+#include "phi_schedule.h"
 
 namespace crysscft {
 
@@ -280,14 +281,8 @@ __global__ void phi_fused_finish_kernel(const double* acc, const T* q,
     }
 }
 
-// phi from the sums of contour_any_kernel: acc[parity][block][point], contour order (null: no slot
-// went there), plus the slots `sp` that the sums leave out, with the trapezoid weights of
-// integrate_phi.
-struct PhiSlots {
-    const double* acc[2][2];
-    int count;
-    long long s[8];
-};
+// phi from the sums of the step launches and the slots that they leave out, with the trapezoid
+// weights of integrate_phi.
 template <typename T>
 __global__ void phi_step_finish_kernel(const T* q, const T* qc,
                                        double* phiA, double* phiB, const IterState* st,
