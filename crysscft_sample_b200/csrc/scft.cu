@@ -1669,7 +1669,7 @@ struct scft_diblock_s {
                                contour_alt_kernel_f32_for(nx, o->eo_f32[0], &smem) != nullptr;
             if (!tiled && force_form <= 1 && solver->simt_steps_f32()) {
                 simt_f32 = true;
-                if (any_phi() && phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
+                if (any_phi()) CKR(make_phi_acc());
                 return SCFT_OK;
             }
         }
@@ -1679,7 +1679,7 @@ struct scft_diblock_s {
             step_fn_f32 = contour_step_kernel_f32_for(nx, o->eo_f32[0], &step_smem_f32);
             if (step_fn_f32) {
                 if (!f_xch.p) CKR(f_xch.alloc(4 * M));
-                if (any_phi() && phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
+                if (any_phi()) CKR(make_phi_acc());
                 return SCFT_OK;
             }
         }
@@ -1693,7 +1693,7 @@ struct scft_diblock_s {
         // fused phi sums: two more tiles (the other chain's FP32 tile, the FP64 products)
         // where they fit (AltShapeF::SMEM_FUSED)
         const size_t smem_fused = smem + (size_t)nx * nx * (sizeof(float) + sizeof(double));
-        f32_phi_fused = fused_phi && U % 2 == 0 && NsA >= 1 && NsB >= 1 && smem_fused <= (size_t)dev_smem;
+        f32_phi_fused = alt_phi() && smem_fused <= (size_t)dev_smem;
         if (f32_phi_fused) smem = smem_fused;
         CK(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
@@ -1704,6 +1704,7 @@ struct scft_diblock_s {
         persistent_grid = 2 * nx;
         persistent_smem = smem;
         if (!f_xch.p) CKR(f_xch.alloc(4 * M));
+        if (f32_phi_fused) CKR(make_phi_acc());
         if (flags.n != alt_flag_count(nx)) CKR(flags.alloc(alt_flag_count(nx)));
         if (!ctrl.p) {
             CKR(ctrl.alloc(2));
@@ -1738,7 +1739,6 @@ struct scft_diblock_s {
         const int n = (int)solver->grid_phy[0];
         phi_fused = f32_phi_fused;  // set up with the launch's shared memory size
         if (phi_fused) {
-            if (phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
             a.phi_acc = phi_acc.p;
             a.done = flags.p + 4 * (size_t)n * n;
         }
@@ -1768,7 +1768,7 @@ struct scft_diblock_s {
         any_fp = solver->any_plan(solver->pos_order());
         if (!any_fp.fn) return SCFT_OK;
         if (d_xch.n < 4 * any_fp.x_count) CKR(d_xch.alloc(std::max(4 * M, 4 * any_fp.x_count)));
-        if (any_phi() && phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
+        if (any_phi()) CKR(make_phi_acc());
         return SCFT_OK;
     }
     // Whether contour_any_kernel sums phi itself: up to 2^16 points, where the sums fit into the
@@ -1778,6 +1778,12 @@ struct scft_diblock_s {
     // Not in batch form 1, whose results are those of the batch kernel bit for bit (it leaves phi to
     // the pass).
     bool any_phi() const { return fused_phi && M <= 65536 && force_form == 0; }
+
+    // Whether the alternating kernels sum phi: both chains, U even (the slots the two chains finish
+    // meet on the same layout), both blocks non-empty
+    bool alt_phi() const { return fused_phi && U % 2 == 0 && NsA >= 1 && NsB >= 1; }
+    // With the plan: a capture cannot allocate.
+    int make_phi_acc() { return phi_acc.n == 8 * M ? SCFT_OK : phi_acc.alloc(8 * M); }
 
     int setup_persistent() {
         // nothing of the plan before is left, whichever way this returns
@@ -1826,6 +1832,7 @@ struct scft_diblock_s {
         }
         if (d_xch.n < 4 * M) CKR(d_xch.alloc(4 * M));
         if (alternating && flags.n != alt_flag_count(nx)) CKR(flags.alloc(alt_flag_count(nx)));
+        if (alternating && alt_phi()) CKR(make_phi_acc());
         CK(cudaFuncSetAttribute(contour_fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, contour_fn, kContourThreads, smem));
@@ -1873,11 +1880,8 @@ struct scft_diblock_s {
         a.spin_limit = spin_limit;
         a.flags = flags.p;
         CK(cudaMemsetAsync(ctrl.p, 0, sizeof(unsigned), st));
-        // phi summed inside the alternating kernel: both chains, U even (the slots the two
-        // chains finish meet on the same layout), both blocks non-empty
-        phi_fused = alternating && fused_phi && U % 2 == 0 && NsA >= 1 && NsB >= 1;
+        phi_fused = alternating && alt_phi();
         if (phi_fused) {
-            if (phi_acc.n != 8 * M) CKR(phi_acc.alloc(8 * M));
             a.phi_acc = phi_acc.p;
             a.done = flags.p + 4 * solver->grid_phy[0] * solver->grid_phy[0];
         }
@@ -2731,6 +2735,7 @@ static int diblock_prepare(scft_diblock_t d, bool want_graph) {
         if (d->graph) cudaGraphDestroy(d->graph);
         d->gexec = nullptr;
         d->graph = nullptr;
+        d->use_graph = true;  // a capture refused was one of the plan before
         CKR(d->setup_persistent());
         d->captured_gen = d->solver->ops_gen;
     }

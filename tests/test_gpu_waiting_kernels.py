@@ -9,7 +9,7 @@ the step launches, which do the same arithmetic.
 import numpy as np
 import pytest
 
-from crysscft_sample_b200 import fields, scft, solvers
+from crysscft_sample_b200 import batch, fields, scft, solvers
 from oracle import scft_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -84,3 +84,19 @@ def test_step_launches_sum_phi_themselves(gpu, kind, N, precision):
     assert np.abs(a["F"] - b["F"]).max() <= 1e-13 * np.abs(b["F"]).max()
     for k in ("phiA", "phiB"):
         assert np.abs(a[k] - b[k]).max() <= 1e-13
+
+
+# the buffer of the sums is there before the batch is captured
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("form", [0, 1])
+def test_a_batch_with_its_own_limit(gpu, precision, form):
+    N = (32, 32, 32)
+    w, h = _fields("PMMM", N), []
+    for limit in (20_000_000, LIMIT):
+        B = batch.BatchSCFT("PMMM", [{"N": N, "L": CELL[0], "fA": FA, "xN": XN}], ds=DS, precision=precision)
+        B.configure(1, form)
+        B.set_wait_limit(limit)
+        B.set_fields(0, *w)
+        h.append(B.iterate(2)["F"])
+        B.close()
+    assert np.abs(h[1] - h[0]).max() <= 1e-12 * np.abs(h[0]).max()
