@@ -326,6 +326,38 @@ def grid256_leg(local: int, stream, steps: int = 10):
     return out
 
 
+def phi_form_leg(device, stream, steps=200):
+    """FP64 iterations/s with phi summed in the contour's launches (up to 65536 points, the default
+    there) against the separate pass over the stored contour, on a 64^3 full grid."""
+    from crysscft_sample_b200 import fields, scft, solvers
+
+    import torch
+
+    N, L = (64, 64, 64), WORKLOAD["L"]
+    G = solvers.make_solver("PMMM", N, device=device)
+    G.set_stream(stream)
+    G.set_cell_para((L, L, L))
+    run = scft.DiblockSCFT(G, WORKLOAD["fA"], WORKLOAD["ds"], WORKLOAD["xN"], WORKLOAD["acc"])
+    w = [fields.to_physical("PMMM", v) for v in fields.seed_fields(N, L, WORKLOAD["phase"])]
+    out = {"workload": "AB diblock BCC 64^3 full grid, PMMM solver on 32^3, Ns=200", "unit": "iterations/s", "steps": steps}
+    F = []
+    for name, fused in (("in_the_contour", True), ("separate_pass", False)):
+        run.set_phi_form(fused)
+        run.set_fields(*w)
+        run.iterate(3)
+        run.set_fields(*w)
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record(stream)
+        F.append(run.iterate(steps)["F"][-1])
+        e1.record(stream)
+        e1.synchronize()
+        out[name] = {"value": steps / (e0.elapsed_time(e1) / 1e3)}
+    out["F_rel_diff_last"] = float(abs(F[1] - F[0]) / abs(F[0]))
+    run.close()
+    G.close()
+    return out
+
+
 def run_ours(args):
     import numpy as np
     import torch
@@ -419,25 +451,6 @@ def run_ours(args):
                                     "iterations from the same fields (the target is stated on the protocol)"),
                       "device_ms": prec_ms_all}
     run.set_precision(args.precision)
-    # the FP64 iterations with phi integrated in a separate pass over the stored contour
-    # instead of inside the contour kernel (same fields, its own warmed-up graph)
-    sep_run = scft.DiblockSCFT(solver, WORKLOAD["fA"], WORKLOAD["ds"], WORKLOAD["xN"], WORKLOAD["acc"])
-    sep_run.set_phi_form(False)
-    sep_run.set_fields(start_fields["wA"], start_fields["wB"])
-    sep_run.iterate(max(args.warmup, 3))
-
-    def separate_phi():
-        sep_run.set_fields(start_fields["wA"], start_fields["wB"])
-        return sep_run.iterate(args.steps)
-
-    hsep, sep_ms = timed(separate_phi)
-    sep_run.close()
-    sep_ms = max_over_ranks(sep_ms)
-    phi_form = {"fused_iterations_per_s": world * args.steps / (fp64_ms_all / 1e3),
-                "separate_pass_iterations_per_s": world * args.steps / (sep_ms / 1e3),
-                "F_rel_diff_last": float(abs(hsep["F"][-1] - href["F"][-1]) / abs(href["F"][-1])),
-                "what": "FP64 iterations: phi summed inside the contour kernel (default) against the "
-                        "separate integrate_phi pass over the stored contour"}
     ms = max_over_ranks(ms)
     value = world * args.steps / (ms / 1e3)
     launches = run.launches_per_iteration()
@@ -450,12 +463,12 @@ def run_ours(args):
     phases_other = run.time_phases(10)
     run.set_precision(args.precision)
     phases = run.time_phases(10)
-    chain_s = phases[1] / 1e3  # one launch of the contour kernel = all 2U triplets of an iteration
+    chain_s = phases[1] / 1e3  # all 2U triplets of an iteration
     b = 8 if args.precision == "fp64" else 4
     fp32_chain_s = (phases_other if args.precision == "fp64" else phases)[1] / 1e3
     fp32_bytes = 2 * U * 3 * M * 4
     precision_form["contour_kernel_fp32"] = {
-        "launch_ms": fp32_chain_s * 1e3, "algorithmic_bytes_per_launch": fp32_bytes,
+        "ms_per_iteration": fp32_chain_s * 1e3, "algorithmic_bytes_per_iteration": fp32_bytes,
         "achieved_gbs": fp32_bytes / fp32_chain_s / 1e9,
         "phases_ms_per_iteration": dict(zip(("total", "triplets", "q_phi", "fields_energy"),
                                             phases_other if args.precision == "fp64" else phases))}
@@ -467,17 +480,17 @@ def run_ours(args):
     if args.grid == 128 and args.solver == "PMMM" and not args.no_extra_legs:
         extra["batch_form"] = batch_leg(local)
         extra["grid256"] = grid256_leg(local, stream)
+        extra["phi_form"] = phi_form_leg(local, stream)
     # per triplet: read q(s), read exp(-w ds/2), write q(s+1); K generated on chip, not counted
-    alg_bytes_launch = 2 * U * 3 * M * b
-    achieved = alg_bytes_launch / chain_s / 1e9
-    # FP64 multiply-adds the triplet kernels execute per point and axis: n/2 with the
-    # even/odd operators, 3n/8 with two even/odd levels (PMMM, 64 or 128 points on every
-    # axis), else n
+    alg_bytes = 2 * U * 3 * M * b
+    achieved = alg_bytes / chain_s / 1e9
+    # FP64 multiply-adds the block forms execute per point and axis (cubic grids): n/2 with the
+    # even/odd halves, on 64, 96 and 128 points 3n/8 with two levels (PMMM, 3M) and n/4 with the
+    # four blocks of a circulant (P1); longer axes run FFT passes, counted as the dense n
     n_phy = solver.get_grid_size_phy()
-    two_level = args.solver == "PMMM" and n_phy[0] in (64, 128) and all(v == n_phy[0] for v in n_phy)
-    per_point = sum((3 * v // 8) if two_level else (v // 2) if (args.solver != "3M" and v % 16 == 0) else v
+    per_point = sum(v if v > 128 else v / 2 if v not in (64, 96, 128) else v / 4 if args.solver == "P1" else 3 * v / 8
                     for v in n_phy)
-    flops_launch = 2.0 * 2 * U * M * per_point
+    flops = 2.0 * 2 * U * M * per_point
     import ctypes as _ct
 
     from crysscft_sample_b200 import _lib as _L
@@ -490,7 +503,7 @@ def run_ours(args):
         with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
             tj = json.load(f)
         key = f"{args.solver}_{args.precision}_{n}"
-        traffic = tj.get(key, {}).get("dram_bytes_per_launch")
+        traffic = tj.get(key, {}).get("dram_bytes_per_iteration")
     except Exception:
         pass
 
@@ -529,15 +542,16 @@ def run_ours(args):
                                         "fields_energy": phases[3]},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic,
-                         "kernel": "contour kernel: one launch = the 2 x 200 triplets of one iteration",
-                         "algorithmic_bytes_per_launch": alg_bytes_launch,
-                         "launch_ms": chain_s * 1e3,
+                         "kernel": "contour launches of one iteration: its 2 x 200 triplets (achieved and traffic "
+                                   "are sums over them)",
+                         "algorithmic_bytes_per_iteration": alg_bytes,
+                         "contour_ms_per_iteration": chain_s * 1e3,
                          "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)" if peak_src == "measured"
                          else "fallback 6650 GB/s",
-                         "fp64": {"achieved_tflops": flops_launch / chain_s / 1e12,
+                         "fp64": {"achieved_tflops": flops / chain_s / 1e12,
                                   "peak_tflops": tens.value, "peak_simt_tflops": simt.value,
-                                  "frac": flops_launch / chain_s / 1e12 / tens.value,
-                                  "flops_per_launch": flops_launch,
+                                  "frac": flops / chain_s / 1e12 / tens.value,
+                                  "flops_per_iteration": flops,
                                   "peak_source": "measured live (scft_measure_fp64_peak, FP64 m8n8k4 MMA)"}
                          if args.precision == "fp64" else None},
             "e2e": {"value": e2e_value, "unit": "iterations/s", "h2d_bytes_per_step": 2 * M * 8,
@@ -546,7 +560,6 @@ def run_ours(args):
                        "samples": clk["samples"]},
             "F_last": float(hist["F"][-1]),
             "precision_form": precision_form,
-            "phi_form": phi_form,
             "drop_in": drop_in,
             **extra,
         }
