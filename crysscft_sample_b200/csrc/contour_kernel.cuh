@@ -16,6 +16,11 @@
 // Grid barriers count arrivals on a counter that the host zeroes before each launch;
 // every wait is bounded (spin limit), after which the kernel records an error and
 // returns, so a lost block can never hang the GPU.
+//
+// Iterations on operators with the reflection symmetry launch one kernel per step instead
+// (contour_step.cuh).  The kernels here run 3m mirrors on grid points (operators without the
+// symmetry), batch form 2, and contexts with a poll limit of their own, which ask for kernels
+// that can time out.
 #pragma once
 #include <cuda.h>  // CUtensorMap (type only)
 #include <cuda_runtime.h>

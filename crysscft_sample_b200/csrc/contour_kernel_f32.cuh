@@ -7,6 +7,9 @@
 // into hi = tf32(x) and lo = tf32(x - hi) and a*b ~ a_lo b_hi + a_hi b_lo + a_hi b_hi,
 // which keeps FP32-level accuracy (the dropped a_lo b_lo term is ~2^-22 relative).
 // Operators are split on the host; field values are split on the fly.
+//
+// Iterations run the same tile operations one launch per phase (contour_step_f32.cuh); the
+// persistent kernel here runs batch form 2 and contexts with a poll limit of their own.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -415,7 +415,7 @@ AxisFftFn<R> axis_fft_kernel_for(int n, int nf, int ext, size_t* smem) {
 }
 
 // Which form runs the per-axis passes: CRYSSCFT_AXIS_FORM=fft or =dense forces one (for
-// measurements and tests).  By default FP64 axes of up to kMmaMaxN points take the tensor-core
+// measurements and tests), and turns every form of one launch per step or two off.  By default FP64 axes of up to kMmaMaxN points take the tensor-core
 // passes (axis_mma.cuh), longer ones the FFT where it exists (256-point P1 axes: 0.28 ms a
 // triplet against 2.99 ms by the SIMT GEMMs); FP32 triplets take the FFT where it exists except
 // on the grids of scft_solver_s::tf32_axis_passes.  FP64 per triplet on one B200, three calls of
@@ -1466,14 +1466,16 @@ struct scft_diblock_s {
     size_t step_smem_f32 = 0;
     bool simt_f32 = false;                // FP32 contour by contour_simt_kernel_f32
     scft_solver_s::AnyPlan any_fp;        // FP64 contour by contour_any_kernel (fn null: not)
-    int force_form = 0;                   // 0 auto, 1 alternating, 2 two-phase, 3 per-axis kernels
+    // 0 auto, 1 auto with phi in the separate pass (step launches, or the alternating kernel with a
+    // poll limit of the caller's own), 2 two-phase kernel where there is one, 3 per-axis kernels
+    int force_form = 0;
     int last_form = 0;                    // force_form the current launch plan was built with
     DevBuf<double> d_xch;                 // exchange buffers, 2 x space_size_phy per chain
     DevBuf<unsigned> flags;               // per-unit phase flags of the alternating kernel
-    bool fused_phi = true;                // FP64 alternating kernel sums phi itself (scft_diblock_set_phi_form)
+    bool fused_phi = true;                // the contour kernels sum phi where they can (scft_diblock_set_phi_form)
     bool phi_fused = false;               // the last launch_contour[_f32] ran with the fused phi sums
     bool f32_phi_fused = false;           // the FP32 launch plan has room for them (setup_persistent_f32)
-    DevBuf<double> phi_acc;               // its sums: [chain][block][layout][tile][n^2], 8 x space_size_phy
+    DevBuf<double> phi_acc;               // their sums, 8 x space_size_phy (PhiSlots, phi_fused_finish_kernel)
     int last_iter_precision = -1;         // precision of the iteration whose contour is stored
     DevBuf<double> stress_buf;            // batched temporaries of scft_diblock_stress
     DevBuf<double> stress_part;           // ... and its partial sums
@@ -1648,7 +1650,8 @@ struct scft_diblock_s {
                     a.out[c] = half == 0 ? x[c] : slice[c];
                     a.w[c] = (c == 0 ? s0 : s1 - 1) < (long long)NsA ? wAds : wBds;
                 }
-                // the slab launch of step t - 2, which finished slot t - 1, is two launches back
+                // slot t - 1 was finished by the slab launch of step t - 2, three launches back (when a
+                // launch starts, every launch before its predecessor has completed)
                 if (half == 0) a.phi = phi.of(t + 1);
                 CK(launch_pdl_if(t + half > 0, contour_simt_kernel_f32, (unsigned)(2 * std::max(nx, ny)), kSimtThreads, smem, st, a));
                 ++solver->launches;
@@ -1674,7 +1677,7 @@ struct scft_diblock_s {
             }
         }
         if (nx != ny || ny != nz || o->eo_f32[0] != o->eo_f32[1] || o->eo_f32[1] != o->eo_f32[2]) return SCFT_OK;
-        // (a caller's own poll limit asks for the kernels that wait)
+        // (a caller's own poll limit asks for the kernels that wait, here and in setup_persistent)
         if (force_form <= 1 && spin_limit == kSpinLimit && axis_form_override() == 0) {
             step_fn_f32 = contour_step_kernel_f32_for(nx, o->eo_f32[0], &step_smem_f32);
             if (step_fn_f32) {
@@ -1771,10 +1774,11 @@ struct scft_diblock_s {
         if (any_phi()) CKR(make_phi_acc());
         return SCFT_OK;
     }
-    // Whether contour_any_kernel sums phi itself: up to 2^16 points, where the sums fit into the
-    // wait for the previous launch (16^3 0.186 against 0.202 ms an iteration with the separate
-    // pass, 24^3 0.401 / 0.424, 40^3 1.24 / 1.30); on larger grids they reach into the launch they
-    // wait for (45^3 1.43 / 1.39, 64^3 1.67 / 1.36 ms).
+    // Whether the step launches (FP64 and FP32) sum phi themselves: up to 2^16 points, where the sums
+    // fit into the wait for the previous launch (16^3 0.186 against 0.202 ms an iteration with the
+    // separate pass, 24^3 0.401 / 0.424, 40^3 1.24 / 1.30; 32^3 with 200 steps 0.521 / 0.507, whose
+    // contour fits in L2); on larger grids they reach into the launch they wait for (45^3 1.43 /
+    // 1.39, 64^3 1.67 / 1.36 ms).
     // Not in batch form 1, whose results are those of the batch kernel bit for bit (it leaves phi to
     // the pass).
     bool any_phi() const { return fused_phi && M <= 65536 && force_form == 0; }

@@ -161,12 +161,13 @@ class DiblockSCFT:
             raise ValueError(f"unknown mixing {kind!r}")
 
     def set_wait_limit(self, spins: int = 20_000_000):
-        """Poll limit of the contour kernels' bounded waits (see scft_diblock_set_wait_limit)."""
+        """Poll limit of the persistent contour kernels' bounded waits; any other than the default
+        makes the iterations run those kernels (see scft_diblock_set_wait_limit)."""
         check(_lib.load().scft_diblock_set_wait_limit(self._h, int(spins)))
 
     def set_phi_form(self, fused: bool = True):
-        """Integrate phi inside the whole-contour kernel (True, the default) or in a separate
-        pass over the stored contour (False); see scft_diblock_set_phi_form."""
+        """Integrate phi inside the contour kernels where the grid allows it (True, the default) or
+        in a separate pass over the stored contour (False); see scft_diblock_set_phi_form."""
         check(_lib.load().scft_diblock_set_phi_form(self._h, 1 if fused else 0))
 
     def residuals(self) -> np.ndarray:

@@ -212,10 +212,13 @@ int scft_diblock_set_mixing(scft_diblock_t d, int history, double beta);
 /* Poll limit of every bounded wait inside the persistent contour kernels (release flags, grid
  * barriers, tile loads; default 20,000,000, about a second).  A wait that runs out makes
  * the kernel record an error, let its own copies land and return, and the iteration call
- * returns SCFT_ERR_TIMEOUT; the context stays usable.  FP64 iterations on grids of up to 64
- * points a side run one launch per contour step, which waits on nothing; with a limit other
- * than the default they run the persistent kernel where it covers the grid.  No counterpart in the reference
- * (it has no device code); a small limit is how the timeout path is tested. */
+ * returns SCFT_ERR_TIMEOUT; the context stays usable.  Iterations launch one kernel per contour
+ * step, which waits on nothing, on FP64 grids of up to 64 points a side and FP32 cubic grids of
+ * 16, 32, 48 and 64.  With a limit other than the default those run a persistent kernel instead
+ * (slower; other rounding in FP64): FP64 grids whose sides are multiples of 8, FP32 the same
+ * cubes.  Other FP64 grids then take three axis passes a step.  Grids that run something else
+ * anyway are not affected.  No counterpart in the reference (it has no device code); a small
+ * limit is how the timeout path is tested. */
 int scft_diblock_set_wait_limit(scft_diblock_t d, long long spins);
 
 /* Where the iterations integrate phi_A and phi_B over the contour (integrate_phi,
@@ -223,9 +226,10 @@ int scft_diblock_set_wait_limit(scft_diblock_t d, long long spins);
  * contour kernels add q(s) q+(s) as the second chain reaches each slot, so a short kernel
  * finishes phi instead of a pass over the stored contour; fused = 0 always uses that
  * separate pass.  The two agree to rounding (the sums run in a different order).  The
- * fused form applies to FP64 grids of up to 65536 physical points and to the alternating
- * whole-contour kernels with an even number of contour steps; other plans use the
- * separate pass either way.  No counterpart in the reference (a form switch of this library). */
+ * fused form applies to the step launches of both precisions on grids of up to 65536 physical
+ * points and, with a wait limit of the caller's own, to the persistent kernels on cubic grids
+ * with an even number of contour steps; other plans, and the step launches and teams of batches in
+ * form 1 or 4, use the separate pass either way.  No counterpart in the reference (a form switch of this library). */
 int scft_diblock_set_phi_form(scft_diblock_t d, int fused);
 
 /* rms residual sqrt(<r, r> / 2M) of each iteration of the last scft_diblock_iterate
@@ -284,8 +288,9 @@ int scft_batch_get_fields(scft_batch_t b, size_t i, double* phiA, double* phiB, 
 /* n_iter iterations of every instance; F and maxinc (may be NULL) get n_iter x n values,
  * iteration-major. */
 int scft_batch_iterate(scft_batch_t b, size_t n_iter, double* F, double* maxinc);
-/* Worker streams and contour-kernel form (0 automatic, 1 alternating layout, 2 two-phase,
- * 3 per-axis kernels, 4 one persistent launch: the contours of every FP64 instance on a cubic
+/* Worker streams and contour-kernel form (0 automatic, 1 the same with phi in the separate pass,
+ * 2 two-phase kernel where there is one, else per-axis kernels, 3 per-axis kernels, 4 one
+ * persistent launch: the contours of every FP64 instance on a cubic
  * grid with a side of 8, 16, .. 64 points run together in one cooperative launch, each chain
  * on a team of CTAs that own several x-planes / y-slabs each; the other instances keep
  * their own kernels).  Forms 0-3 launch each instance's own contour kernels. */
