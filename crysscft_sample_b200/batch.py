@@ -13,7 +13,7 @@ from ._lib import check
 
 __all__ = ["BatchSCFT", "batch_config", "FORMS"]
 
-FORMS = {0: "automatic", 1: "alternating layout", 2: "two-phase", 3: "per-axis kernels",
+FORMS = {0: "automatic", 1: "automatic, phi in the separate pass", 2: "two-phase", 3: "per-axis kernels",
          4: "one persistent launch (team kernel)"}
 
 

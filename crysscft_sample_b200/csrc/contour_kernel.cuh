@@ -18,8 +18,8 @@
 // returns, so a lost block can never hang the GPU.
 //
 // Iterations on operators with the reflection symmetry launch one kernel per step instead
-// (contour_step.cuh).  The kernels here run 3m mirrors on grid points (operators without the
-// symmetry), batch form 2, and contexts with a poll limit of their own, which ask for kernels
+// (contour_step.cuh).  The kernels here run 3m with shifted mirror planes (operators without
+// the symmetry), batch form 2, and contexts with a poll limit of their own, which ask for kernels
 // that can time out.
 #pragma once
 #include <cuda.h>  // CUtensorMap (type only)
